@@ -9,9 +9,10 @@ estimate, at a profile, sample format, frame size and precision.  `listed` gives
 The Basic and the Final estimate are separate cases, the Final one on a ref clip made here: its
 match lists follow its ref, so behind a Basic estimate, whose sums are atomics in any order, a
 last-bit difference swaps near-equal matches and the outputs of two runs could not be compared.
-For the same reason the filters' integer clips are 16-bit (8-bit ones take the same path, but two
-runs differ in none to a handful of their pixels, too few to tell runs apart by); conversions are
-exact and are drawn in 8 bits too.
+Integer clips take the conversion kernels and then the same path as float ones.  They appear where
+two runs differ in enough of the rounded pixels to be told from a fault: 16-bit Basic and V-BM3D
+requests, whose sums differ in thousands of pixels from run to run; 8-bit outputs and Final's
+16-bit ones differ in none to a few dozen.  Conversions are exact and are drawn in every format.
 """
 import ctypes as C
 import math
@@ -41,8 +42,8 @@ def listed():
     return [
         # one small gray picture at every default (profile "fast"): launch and host latency
         _case("basic_fast_cif", "basic", "GRAY", "f32", 352, 288, 1, "fast", 10.0),
-        # a standard-definition 16-bit frame, refined in the default profile
-        _case("final_fast_sd_u16", "final", "YUV", "u16", 720, 480, 1, "fast", 10.0),
+        # a standard-definition frame, refined in the default profile
+        _case("final_fast_sd", "final", "YUV", "f32", 720, 480, 1, "fast", 10.0),
         # a VapourSynth script: one 16-bit frame in host memory in, the estimate in host memory out
         _case("basic_lc_hd_host_u16", "basic", "YUV", "u16", 1280, 720, 1, "lc", 10.0, host=True),
         # one 1080p frame on the GPU, refined at the normal profile
@@ -91,7 +92,7 @@ def draw(rng):
         return _case("", kind, rng.choice(["GRAY", "YUV", "OPP"]), rng.choice(["u16", "u16", "f32"]), width, height, frames,
                      rng.choice(["fast", "lc", "np"]), sigma, out=rng.choice(["stacked16", "aggregate16", "aggregate32"]))
     profile = rng.choice(["fast", "fast", "lc", "np", "np", "high", "vn"])
-    return _case("", kind, rng.choice(["GRAY", "YUV", "OPP", "RGB"]), rng.choice(["u16", "u16", "f32", "f32"]), width, height,
+    return _case("", kind, rng.choice(["GRAY", "YUV", "OPP", "RGB"]), rng.choice(["u16", "f32"] if kind == "basic" else ["f32"]), width, height,
                  frames, profile, 40.0 if profile == "vn" else sigma, host=rng.random() < 0.2)
 
 
