@@ -39,6 +39,27 @@ BM3D_HD inline int vbm_warp_floats(int sp_cap, int list_cap, int G, int ps_num, 
     return 2 * sp_cap + vbm_tmp_cap(sp_cap) + 4 * list_cap + 2 * G + ps_num + B * B;
 }
 
+// vbm_predict8_kernel: the window of a centre (2 range + 8 rows and columns) fits a warp's 32 lanes
+constexpr int kPsMaxRange = 12;
+BM3D_HD inline int vbm8_pitch(int range) { return 2 * range + 9; }   // odd: lanes on consecutive rows
+BM3D_HD inline int vbm8_patch_floats(int range) { return ((2 * range + 8) * vbm8_pitch(range) + 7) & ~3; }
+// per warp: a work region -- two window patches and the lanes' distances (four candidates per lane
+// and round), or sp, tmp and sk of a search redone by the general routines, or the keys of the
+// concatenated list in lane columns ...
+BM3D_HD inline int vbm8_work_floats(int range, int sp_cap, int list_cap)
+{
+    const int span = 2 * range + 1, rounds = (2 * span * ((span + 3) / 4) + 31) / 32;
+    int n = 2 * vbm8_patch_floats(range) + rounds * 128;
+    if (n < 3 * vbm_tmp_cap(sp_cap)) n = 3 * vbm_tmp_cap(sp_cap);
+    if (n < list_cap + 32) n = list_cap + 32;
+    return (n + 3) & ~3;
+}
+// ... after the reference block; then the list (keys, positions), a frame's selection, two centres
+BM3D_HD inline int vbm8_warp_floats(int range, int sp_cap, int list_cap, int G)
+{
+    return (64 + vbm8_work_floats(range, sp_cap, list_cap) + 2 * list_cap + 2 * G + 2 + 3) & ~3;
+}
+
 // Precision-form block matching (bm_tc_kernel): at most kBmtRefs reference blocks per CTA and
 // kBmtCols candidate columns (the union of their search windows along the row).
 constexpr int kBmtRefs = 8;

@@ -1691,15 +1691,21 @@ public:
         va.desc = dwin;
         va.desc_frame = (long long)(W - 7) * (H - 7);
         va.nprop = kLearnedFrameProposals;
+        // the register-blocked kernel takes the default form of the search (8 x 8 blocks, step 1, at
+        // most two centres); others, and windows beyond a warp's width, take the general kernel
+        const bool fast_ps = para.B == 8 && para.psstep == 1 && para.psnum <= 2 && para.G <= 32 && !dwin &&
+                             va.ps_range <= kPsMaxRange;
         size_t smem = 0;
         int warps = 4;
         for (; warps >= 1; warps /= 2) {
-            smem = sizeof(float) * (size_t)warps * vbm_warp_floats(va.sp_cap, va.list_cap, va.G, va.ps_num, va.B);
+            smem = sizeof(float) * (size_t)warps *
+                   (fast_ps ? vbm8_warp_floats(va.ps_range, va.sp_cap, va.list_cap, va.G)
+                            : vbm_warp_floats(va.sp_cap, va.list_cap, va.G, va.ps_num, va.B));
             if (smem <= 200 * 1024) break;
         }
         if (warps < 1) return fail(BM3D_ERR_UNSUPPORTED, err("ps_num / ps_range too large for the predictive-search buffers"));
         va.warps = warps;
-        CU(launch_vbm_predict(va, rc, smem, stream));
+        CU(launch_vbm_predict(va, fast_ps, rc, smem, stream));
         mark(3);
         // K3+K4 into the accumulators
         for (int p = 0; p < np; ++p)

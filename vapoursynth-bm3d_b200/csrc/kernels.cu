@@ -140,11 +140,17 @@ cudaError_t launch_bm_full(const BMArgs &a, int nframes, size_t smem, cudaStream
     return cudaGetLastError();
 }
 
-cudaError_t launch_vbm_predict(const VBMArgs &a, int nframes, size_t smem, cudaStream_t s)
+cudaError_t launch_vbm_predict(const VBMArgs &a, bool fast, int nframes, size_t smem, cudaStream_t s)
 {
     dim3 grid((a.nbx + a.warps - 1) / a.warps, a.nby, nframes);
     dim3 block(32 * a.warps);
     cudaError_t e;
+    if (fast) {
+        if ((e = allow_smem(vbm_predict8_kernel, smem)) != cudaSuccess) return e;
+        COUNT_LAUNCH();
+        vbm_predict8_kernel<<<grid, block, smem, s>>>(a);
+        return cudaGetLastError();
+    }
     if ((e = allow_smem(vbm_predict_kernel, smem)) != cudaSuccess) return e;
     COUNT_LAUNCH();
     vbm_predict_kernel<<<grid, block, smem, s>>>(a);

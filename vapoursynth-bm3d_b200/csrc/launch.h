@@ -32,7 +32,9 @@ cudaError_t launch_bm_learned(const BMArgs &a, const void *desc, int nprop, int 
 // Precision-form full search (B = 8, candidate step 1, group size <= 32, search windows of
 // L.nrc consecutive reference blocks within 64 candidate columns): same lists as launch_bm_full.
 cudaError_t launch_bm_tc(const BMArgs &a, const BmtLayout &L, int nframes, cudaStream_t s);
-cudaError_t launch_vbm_predict(const VBMArgs &a, int nframes, size_t smem_bytes, cudaStream_t s);
+// fast: the register-blocked kernel (B = 8, ps_step 1, ps_num <= 2, G <= 32, no descriptors,
+// ps_range <= kPsMaxRange); same lists
+cudaError_t launch_vbm_predict(const VBMArgs &a, bool fast, int nframes, size_t smem_bytes, cudaStream_t s);
 // Fast collaborative filter (B = 8, G in {8, 16, 32}, any group length n <= G); sizes its own
 // grid (one CTA per run of consecutive groups); returns cudaErrorInvalidValue for other shapes.
 cudaError_t launch_cf_fast(const CFArgs &a, cudaStream_t s);
