@@ -174,6 +174,16 @@ struct CFArgs {
     int *retained;
 };
 
+// Tiles of reference blocks of cf_box_kernel and the shared-memory box they need.
+struct CFBox {
+    const int *scan_y, *scan_x;
+    int nby, nbx, range;       // range: no list entry is further than this from its reference block,
+                               // except the block at (0, 0)
+    int tx, ty;                // tiles along a row and along a column of reference blocks
+    int rows, pitch;           // box rows and row pitch in cells
+    int plane[3], nplanes;     // processed planes
+};
+
 struct VBMArgs {
     const float *ref;             // reference Y planes of the clip window workspace
     long long frame_stride;

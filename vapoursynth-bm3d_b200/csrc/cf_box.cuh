@@ -1,0 +1,526 @@
+// cf_box.cuh -- K3+K4, plain form: the collaborative filter of B = 8 groups with the image region of
+// a tile of groups held in shared memory.
+//
+// A CTA takes one plane of a tile of neighbouring reference blocks.  Every block their lists
+// can name lies in one box of the image, the union of their search windows, or is the block at (0, 0)
+// (the reference's trailing candidate), which gets a slot of its own beside the box.  The box is
+// copied to shared memory once, the groups' blocks are read from there, and their estimates are added
+// into a second box in fixed point, which goes to the numerator plane once, with vector atomics.
+// Shared-memory atomics are native for 32-bit integers only (float and 64-bit ones are compare-and-swap
+// loops, 437 clocks a block and warp against 100), so a cell is two words of its own: a term is split
+// exactly into a multiple of 2^-13 and a multiple of 2^-32.
+//
+// Final (cf_box_kernel): a pair of warps per slot of 32 blocks (32 / G groups), both filtering the
+// reference and the source blocks at once as the halves of packed fp32 pairs (one instruction for
+// both, each half rounded as the scalar instruction would).  2-D transforms: two lanes per block, four
+// rows each, exchanged by shuffles for the columns; z stage: lane = coefficient column of the transpose
+// buffer; the estimates are inverted and scattered by the warp that holds their blocks.
+// The arithmetic is that of common.cuh's transforms, operation for operation, as in cf_fast_kernel.
+// Bound: the FP32 pipe (9.9 k clocks of a step's 19 k; the transforms are separable butterflies, and a
+// packed instruction takes the pipe twice) and, in the phases that do not use it, the latency of 16
+// warps per SM, which the transpose buffers and 128 registers a thread allow.  1920x1080 RGB x 8,
+// G = 32: 120.3 ms with one warp per group, gathers from global memory and a 64-bit box, 47.9 ms now.
+#pragma once
+
+#include "cf.cuh"
+#include "tc.cuh"
+
+namespace bm3d {
+
+// Fixed point: units of the high and the low word.  A pixel takes at most 128 groups x 32 blocks = 2^12
+// terms per tile; terms below 2^6 keep the high word below 2^31 and the low one below 2^30, larger ones
+// go to the plane directly.
+constexpr float kBoxMax = 64.0f;
+constexpr float kBoxHi = 8192.0f, kBoxHiUnit = 1.220703125e-4f;               // 2^13, 2^-13
+constexpr float kBoxLo = 4294967296.0f, kBoxLoUnit = 2.3283064365386963e-10f;  // 2^32, 2^-32
+constexpr float kBoxRound = 12582912.0f;                                       // 1.5 x 2^23: rounds to an integer
+constexpr int kBoxRoundBits = 0x4b400000;
+
+// sum of a cell's words as a float
+__device__ __forceinline__ float box_value(int hi, int lo)
+{
+    // carry into the high word; both words are then exact in fp32 (the high one below 2^24 units)
+    return __fmaf_rn(__int2float_rn(lo & 0x7ffff), kBoxLoUnit, __int2float_rn(hi + (lo >> 19)) * kBoxHiUnit);
+}
+
+__device__ __forceinline__ void pair_barrier(int id) { asm volatile("bar.sync %0, 64;" ::"r"(id) : "memory"); }
+
+using tc::f2;
+using tc::pk;
+using tc::upk;
+using tc::fma2;
+
+__device__ __forceinline__ f2 add2(f2 a, f2 b)
+{
+    f2 r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+
+// Product of both halves by scalar multiplications, for a product that a packed sum follows: a packed
+// one would be contracted with the sum into one rounding
+__device__ __forceinline__ f2 mul2s(f2 v, float c)
+{
+    float a, b;
+    upk(v, a, b);
+    return pk(__fmul_rn(a, c), __fmul_rn(b, c));
+}
+
+// Outputs formed together: their chains of dependent multiply-adds run side by side
+constexpr int kChains = 4;
+
+// fdct_reg on packed pairs; outputs are handed to f(k, step, X) in sets as they are produced (X[i] is
+// output k + i * step), the odd ones of the longest level first, so that a column's inputs are dead
+// before its spectrum is complete
+template <int N, int S = 1, class F>
+__device__ __forceinline__ void fdct2(const f2 (&x)[N], F &&f)
+{
+    if constexpr (N == 2) {
+        const f2 X[2] = {tc::mul2(add2(x[0], x[1]), pk(2.0f, 2.0f)), mul2s(sub2(x[0], x[1]), odd_coef(2, 0, 0))};
+        f(0, S, X);
+    } else if constexpr (N == 1) {
+        const f2 X[1] = {tc::mul2(x[0], pk(2.0f, 2.0f))};
+        f(0, S, X);
+    } else {
+        constexpr int h = N / 2, C = h < kChains ? h : kChains;
+        f2 e[h], o[h];
+#pragma unroll
+        for (int j = 0; j < h; ++j) {
+            e[j] = add2(x[j], x[N - 1 - j]);
+            o[j] = sub2(x[j], x[N - 1 - j]);
+        }
+#pragma unroll
+        for (int m = 0; m < h; m += C) {
+            f2 X[C];
+#pragma unroll
+            for (int i = 0; i < C; ++i) X[i] = tc::mul2(o[0], pk(odd_coef(N, m + i, 0), odd_coef(N, m + i, 0)));
+#pragma unroll
+            for (int j = 1; j < h; ++j)
+#pragma unroll
+                for (int i = 0; i < C; ++i) X[i] = fma2(o[j], pk(odd_coef(N, m + i, j), odd_coef(N, m + i, j)), X[i]);
+            f((2 * m + 1) * S, 2 * S, X);
+        }
+        fdct2<h, 2 * S>(e, f);
+    }
+}
+
+// idct_reg on packed pairs
+template <int N>
+__device__ __forceinline__ void idct2(const f2 (&X)[N], f2 (&y)[N])
+{
+    if constexpr (N == 2) {
+        const f2 o = mul2s(X[1], odd_coef(2, 0, 0));
+        y[0] = add2(X[0], o);
+        y[1] = sub2(X[0], o);
+    } else {
+        constexpr int h = N / 2;
+        f2 ev[h], E[h], o[h];
+#pragma unroll
+        for (int m = 0; m < h; ++m) ev[m] = X[2 * m];
+        idct2<h>(ev, E);
+#pragma unroll
+        for (int k = 0; k < h; ++k) o[k] = tc::mul2(X[1], pk(odd_coef(N, k, 0), odd_coef(N, k, 0)));
+#pragma unroll
+        for (int m = 1; m < h; ++m)
+#pragma unroll
+            for (int k = 0; k < h; ++k) o[k] = fma2(X[2 * m + 1], pk(odd_coef(N, k, m), odd_coef(N, k, m)), o[k]);
+#pragma unroll
+        for (int k = 0; k < h; ++k) {
+            y[k] = add2(E[k], o[k]);
+            y[N - 1 - k] = sub2(E[k], o[k]);
+        }
+    }
+}
+
+// idct_reg with kChains outputs side by side, handed to f(k, y_k)
+template <int N, class F>
+__device__ __forceinline__ void idct_sets(const float (&X)[N], F &&f)
+{
+    if constexpr (N == 1) {
+        f(0, X[0]);
+    } else {
+        constexpr int h = N / 2, C = h < kChains ? h : kChains;
+        float ev[h], E[h];
+#pragma unroll
+        for (int m = 0; m < h; ++m) ev[m] = X[2 * m];
+        idct_sets<h>(ev, [&](int k, float v) { E[k] = v; });
+#pragma unroll
+        for (int k = 0; k < h; k += C) {
+            float o[C];
+#pragma unroll
+            for (int i = 0; i < C; ++i) o[i] = __fmul_rn(X[1], odd_coef(N, k + i, 0));
+#pragma unroll
+            for (int m = 1; m < h; ++m)
+#pragma unroll
+                for (int i = 0; i < C; ++i) o[i] = __fmaf_rn(X[2 * m + 1], odd_coef(N, k + i, m), o[i]);
+#pragma unroll
+            for (int i = 0; i < C; ++i) {
+                f(k + i, __fadd_rn(E[k + i], o[i]));
+                f(N - 1 - k - i, __fsub_rn(E[k + i], o[i]));
+            }
+        }
+    }
+}
+
+// w[i] = r2[i] / (r2[i] + sg): reciprocal estimate, quotient, and one correction by the exact remainder
+// (Markstein, IBM J. Res. Dev. 34, 1990), which rounds as the division does but for quotients within a
+// few 2^-46 of a tie.  The division itself (a dozen instructions and a branch each) serves where the
+// estimate would underflow.
+template <int C>
+__device__ __forceinline__ void wiener_weights(const float (&r2)[C], float sg, float (&w)[C])
+{
+    float d[C], top = 0.0f;
+#pragma unroll
+    for (int i = 0; i < C; ++i) {
+        d[i] = __fadd_rn(r2[i], sg);
+        top = fmaxf(top, d[i]);
+    }
+    if (top < 4.2535296e37f) {            // 2^125
+#pragma unroll
+        for (int i = 0; i < C; ++i) {
+            float y;
+            asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(d[i]));
+            const float q = __fmul_rn(r2[i], y);
+            w[i] = __fmaf_rn(__fmaf_rn(-d[i], q, r2[i]), y, q);
+        }
+    } else {
+#pragma unroll
+        for (int i = 0; i < C; ++i) w[i] = __fdiv_rn(r2[i], d[i]);
+    }
+}
+
+constexpr int kBT = 66;                  // cells between the blocks of the transpose buffer: 2 mod 16, so that
+                                         // eight blocks x two columns, or 16 columns, fall in distinct banks
+
+__device__ __forceinline__ f2 shfl_pair(f2 v)
+{
+    float a, b;
+    upk(v, a, b);
+    return pk(__shfl_xor_sync(0xffffffffu, a, 1), __shfl_xor_sync(0xffffffffu, b, 1));
+}
+
+// Block at `b` (pitch P cells) of the box of (reference, source) pairs -> its 2-D coefficients at `t`.
+// Lane half h (lane & 1) transforms rows 0 .. 3 (h = 0) or 7 .. 4 (h = 1), then the columns 2k + h.
+__device__ __forceinline__ void box_forward(const f2 *b, int P, f2 *t, int h)
+{
+    f2 keep[4][4], give[4][4];            // [row][column pair]: columns 2k + h, columns 2k + 1 - h
+    const int step = h ? -P : P;
+    b += h ? 7 * P : 0;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        f2 x[8], X[8];
+#pragma unroll
+        for (int k = 0; k < 8; ++k) x[k] = b[i * step + k];
+        fdct2<8>(x, [&](int k, int st, const auto &v) {
+#pragma unroll
+            for (int c = 0; c < (int)(sizeof(v) / sizeof(v[0])); ++c) X[k + c * st] = v[c];
+        });
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            keep[i][k] = h ? X[2 * k + 1] : X[2 * k];
+            give[i][k] = h ? X[2 * k] : X[2 * k + 1];
+        }
+    }
+    const f2 sg = h ? pk(-1.0f, -1.0f) : pk(1.0f, 1.0f);
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        // first level of the column transform across the two lanes: lane 1's differences, and so its
+        // odd outputs, have the other sign
+        f2 e[4], o[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const f2 v = shfl_pair(give[i][k]);
+            e[i] = add2(keep[i][k], v);
+            o[i] = sub2(keep[i][k], v);
+        }
+        f2 *c = t + 2 * k + h;
+        f2 X[4];
+#pragma unroll
+        for (int m = 0; m < 4; ++m) X[m] = tc::mul2(o[0], pk(odd_coef(8, m, 0), odd_coef(8, m, 0)));
+#pragma unroll
+        for (int j = 1; j < 4; ++j)
+#pragma unroll
+            for (int m = 0; m < 4; ++m) X[m] = fma2(o[j], pk(odd_coef(8, m, j), odd_coef(8, m, j)), X[m]);
+#pragma unroll
+        for (int m = 0; m < 4; ++m) c[(2 * m + 1) * 8] = tc::mul2(X[m], sg);
+        fdct2<4, 2>(e, [&](int y, int st, const auto &v) {
+#pragma unroll
+            for (int i = 0; i < (int)(sizeof(v) / sizeof(v[0])); ++i) c[(y + i * st) * 8] = v[i];
+        });
+    }
+}
+
+// Inverse 2-D transform, scaled, of the filtered coefficients (the low words of the cells) of the block
+// at `t`; the estimates (zeros for a place past the group's end) go to the block's first 64 words, column by column.  Lane half h inverts the
+// columns 2k + h, then the rows 4h .. 4h + 3.
+__device__ __forceinline__ void box_inverse(float *t, float scale, bool active, int h)
+{
+    float keep[4][4], give[4][4];         // [row][column k]
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+        f2 X[8], y[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) X[i] = pk(t[2 * (i * 8 + 4 * q + h)], t[2 * (i * 8 + 4 * q + 2 + h)]);
+        idct2<8>(X, y);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            float a0, a1, b0, b1;
+            upk(y[i], a0, a1);
+            upk(y[i + 4], b0, b1);
+            keep[i][2 * q] = h ? b0 : a0;
+            keep[i][2 * q + 1] = h ? b1 : a1;
+            give[i][2 * q] = h ? a0 : b0;
+            give[i][2 * q + 1] = h ? a1 : b1;
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int k = 0; k < 4; ++k) give[i][k] = __shfl_xor_sync(0xffffffffu, give[i][k], 1);
+    const f2 sc = pk(scale, scale);
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+        f2 X[8], y[8];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            X[2 * k] = pk(h ? give[2 * q][k] : keep[2 * q][k], h ? give[2 * q + 1][k] : keep[2 * q + 1][k]);
+            X[2 * k + 1] = pk(h ? keep[2 * q][k] : give[2 * q][k], h ? keep[2 * q + 1][k] : give[2 * q + 1][k]);
+        }
+        idct2<8>(X, y);
+#pragma unroll
+        for (int k = 0; k < 8; ++k) *reinterpret_cast<f2 *>(t + k * 8 + 4 * h + 2 * q) = active ? tc::mul2(y[k], sc) : 0ull;
+    }
+}
+
+// Wiener z stage of one coefficient column (cells t[z * kBT]) of a group of N blocks: the filtered source
+// column into the cells' low words; returns the sum of the squared weights
+template <int N>
+__device__ __noinline__ float box_wiener(int at, float sg)
+{
+    extern __shared__ __align__(16) float smem[];
+    f2 *t = reinterpret_cast<f2 *>(smem) + at;
+    f2 x[N];
+    float Y[N];
+#pragma unroll
+    for (int z = 0; z < N; ++z) x[z] = t[z * kBT];
+    float l2 = 0.0f;
+    fdct2<N>(x, [&](int k, int st, const auto &v) {
+        constexpr int C = (int)(sizeof(v) / sizeof(v[0]));
+        float r2[C], sv[C], w[C];
+#pragma unroll
+        for (int i = 0; i < C; ++i) {
+            float r;
+            upk(v[i], r, sv[i]);
+            r2[i] = __fmul_rn(r, r);
+        }
+        wiener_weights<C>(r2, sg, w);
+#pragma unroll
+        for (int i = 0; i < C; ++i) {
+            Y[k + i * st] = __fmul_rn(sv[i], w[i]);
+            l2 = __fmaf_rn(w[i], w[i], l2);
+        }
+    });
+    idct_sets<N>(Y, [&](int z, float v) { reinterpret_cast<float *>(t + z * kBT)[0] = v; });
+    return l2;
+}
+
+// the same for a length without an unrolled transform: the direct sums of both columns at once
+__device__ __noinline__ float box_wiener_direct(int at, float sg, int n, const float *fwd, const float *inv)
+{
+    extern __shared__ __align__(16) float smem[];
+    float *t = smem + 2 * at;
+    float R[32], X[32];
+    direct_sums2<2 * kBT>(t, t + 1, fwd, n, true, R, X);
+    float l2 = 0.0f;
+    for (int z = 0; z < n; ++z) {
+        const float r2 = __fmul_rn(R[z], R[z]);
+        const float w = __fdiv_rn(r2, __fadd_rn(r2, sg));
+        l2 = __fadd_rn(l2, __fmul_rn(w, w));
+        t[2 * kBT * z] = __fmul_rn(X[z], w);
+    }
+    direct_sums2<2 * kBT>(t, t, inv, n, false, R, X);
+    for (int z = 0; z < n; ++z) t[2 * kBT * z] = R[z];
+    return l2;
+}
+
+template <int G>
+__device__ __forceinline__ float box_wiener_any(int at, float sg, int n, const CFArgs &a)
+{
+    if (n == G) return box_wiener<G>(at, sg);
+    if (G > 16 && n == 16) return box_wiener<(G > 16 ? 16 : 1)>(at, sg);
+    if (G > 8 && n == 8) return box_wiener<(G > 8 ? 8 : 1)>(at, sg);
+    if (n == 4) return box_wiener<4>(at, sg);
+    if (n == 2) return box_wiener<2>(at, sg);
+    if (n == 1) return box_wiener<1>(at, sg);
+    return box_wiener_direct(at, sg, n, dtab_for(a, n, false), dtab_for(a, n, true));
+}
+
+template <int G, int NP>
+__global__ void __launch_bounds__(NP * 64, 8 / NP) cf_box_kernel(CFArgs a, CFBox g)
+{
+    extern __shared__ __align__(16) float smem[];
+    constexpr int GPW = 32 / G;                     // groups per slot
+    constexpr int kT = 32 * kBT;                    // cells of a transpose buffer
+    const int lane = (int)lane_id();
+    const int warp = threadIdx.x >> 5, pair = warp >> 1, role = warp & 1;
+    const int p = g.plane[blockIdx.y];
+    // tile [bx0, bx1) x [by0, by1) of reference blocks of frame f
+    const int rx = blockIdx.x % g.tx, rest = blockIdx.x / g.tx;
+    const int rr = rest % g.ty, f = rest / g.ty;
+    const int bx0 = (int)((long long)rx * g.nbx / g.tx), bx1 = (int)((long long)(rx + 1) * g.nbx / g.tx);
+    const int by0 = (int)((long long)rr * g.nby / g.ty), by1 = (int)((long long)(rr + 1) * g.nby / g.ty);
+    const int P = g.pitch;
+
+    // the box: rows [y0, y0 + bh), columns [x0, x0 + bw), whole 16-byte chunks; block (0, 0) in 64 cells after it
+    const int y0 = max(0, g.scan_y[by0] - g.range), bh = min(a.H, g.scan_y[by1 - 1] + g.range + 8) - y0;
+    const int x0 = max(0, g.scan_x[bx0] - g.range) & ~3;
+    const int bw = (min(a.W, g.scan_x[bx1 - 1] + g.range + 8) - x0 + 3) & ~3;
+    const int slot0 = g.rows * P, cells = slot0 + 64;
+    f2 *tr = reinterpret_cast<f2 *>(smem);
+    int *acc = reinterpret_cast<int *>(tr + NP * kT);                  // high words, then low words
+    f2 *box = tr + NP * kT + cells;                                             // (reference, source) pairs
+    float *red = reinterpret_cast<float *>(box + cells) + pair * 2 * GPW;   // [group of the slot][warp]
+    const float *src = a.src[p] + f * a.frame_stride, *ref = a.ref[p] + f * a.frame_stride;
+    const int h = lane & 1;
+    const int blk = 16 * role + (lane >> 1);        // the lane's block of a slot: group sub, place z
+    const int sub = blk / G, z = blk - sub * G;
+    // slots run along the tile's rows, GPW groups each
+    const int spr = (bx1 - bx0 + GPW - 1) / GPW, nslots = spr * (by1 - by0);
+    auto slot_at = [&](int slot, int &bx) -> long long {
+        const int sr = slot / spr;
+        bx = bx0 + (slot - sr * spr) * GPW;
+        return ((long long)f * g.nby + by0 + sr) * g.nbx + bx;
+    };
+    // length and z-th position of the lane's group of a slot (n = 0: no such group)
+    auto fetch = [&](int slot, int &n, uint32_t &pos) {
+        n = 0;
+        if (slot >= nslots) return;
+        int bx;
+        const long long grp = slot_at(slot, bx) + sub;
+        if (bx + sub < bx1) {
+            n = a.count[grp];
+            pos = a.pos[grp * G + z];
+        }
+    };
+    int n1 = 0;
+    uint32_t pos1 = 0;
+    fetch(pair, n1, pos1);
+    // all of a thread's loads are in flight together: the staging is one memory latency
+    const int qw = bw >> 2, chunks = bh * qw + 16;
+    for (int e0 = threadIdx.x; e0 < chunks; e0 += 4 * NP * 64) {
+        float4 s4[4], r4[4];
+        int at[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const int e = e0 + k * NP * 64;
+            if (e >= chunks) continue;
+            const int yy = e / qw, c = 4 * (e - yy * qw), m = e - (chunks - 16);
+            const long long go = m < 0 ? (long long)(y0 + yy) * a.ld + x0 + c : (long long)(m >> 1) * a.ld + 4 * (m & 1);
+            at[k] = m < 0 ? yy * P + c : slot0 + 4 * m;
+            s4[k] = __ldg(reinterpret_cast<const float4 *>(src + go));
+            r4[k] = __ldg(reinterpret_cast<const float4 *>(ref + go));
+        }
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            if (e0 + k * NP * 64 >= chunks) continue;
+            float4 *d = reinterpret_cast<float4 *>(box + at[k]);
+            d[0] = make_float4(r4[k].x, s4[k].x, r4[k].y, s4[k].y);
+            d[1] = make_float4(r4[k].z, s4[k].z, r4[k].w, s4[k].w);
+        }
+    }
+    for (int e = threadIdx.x; e < (cells >> 1); e += NP * 64) reinterpret_cast<int4 *>(acc)[e] = make_int4(0, 0, 0, 0);
+    __syncthreads();
+
+    f2 *tb = tr + pair * kT + blk * kBT;
+    const int sy = lane & 7, sx = lane >> 3;        // the lane's pixel of a block in the scatter (and column sx + 4)
+    for (int slot = pair; slot < nslots; slot += NP) {
+        const int n = min(n1, G);
+        // a place past the group's end filters any block of the box and adds zeros
+        const bool active = z < n;
+        const int y = unpack_y(pos1), x = unpack_x(pos1);
+        const bool in = y >= y0 && y + 8 <= y0 + bh && x >= x0 && x + 8 <= x0 + bw;
+        const int off = !active ? 0 : in ? (y - y0) * P + x - x0 : slot0;
+        const uint32_t pos = active ? pos1 : 0u;
+        fetch(slot + NP, n1, pos1);
+        box_forward(box + off, off < slot0 ? P : 8, tb, h);
+        pair_barrier(1 + pair);
+        // z stage: warp `role` takes columns 32 role .. 32 role + 31 of every group of the slot
+        int sbx;
+        const long long sgrp = slot_at(slot, sbx);
+#pragma unroll 1
+        for (int q = 0; q < GPW; ++q) {
+            if (sbx + q >= bx1) break;
+            const int nq = min(a.count[sgrp + q], G);
+            float l2 = box_wiener_any<G>(pair * kT + q * G * kBT + role * 32 + lane, a.wsig2[p][nq - 1], nq, a);
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) l2 = __fadd_rn(l2, __shfl_xor_sync(0xffffffffu, l2, o));
+            if (lane == 0) red[2 * q + role] = l2;
+        }
+        pair_barrier(1 + pair);
+        const float l2 = __fadd_rn(red[2 * sub], red[2 * sub + 1]);
+        const float eps = 1.1920928955078125e-07f;
+        const float denW = __fdiv_rn(1.0f, l2 > eps ? l2 : eps);
+        box_inverse(reinterpret_cast<float *>(tb), active ? __fdiv_rn(denW, a.amp[n - 1]) : 0.0f, active, h);
+        __syncwarp();
+        // aggregation, four blocks per step
+        const float *v = reinterpret_cast<const float *>(tr + pair * kT + 16 * role * kBT) + lane;
+        int *cell = acc + sy * P + sx, *cell0 = acc + sy * 8 + sx;
+#pragma unroll
+        for (int i = 0; i < 16; i += 4) {
+            f2 e[4];
+            int o[4];
+            bool fits = true;
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                o[k] = __shfl_sync(0xffffffffu, off, 2 * (i + k));
+                const float e0 = v[(i + k) * 2 * kBT], e1 = v[(i + k) * 2 * kBT + 32];
+                fits = fits && fabsf(e0) < kBoxMax && fabsf(e1) < kBoxMax;
+                e[k] = pk(e0, e1);
+            }
+            if (__all_sync(0xffffffffu, fits)) {
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    const f2 hi = fma2(e[k], pk(kBoxHi, kBoxHi), pk(kBoxRound, kBoxRound));
+                    const f2 rest = fma2(sub2(hi, pk(kBoxRound, kBoxRound)), pk(-kBoxHiUnit, -kBoxHiUnit), e[k]);
+                    const f2 lo = fma2(rest, pk(kBoxLo, kBoxLo), pk(kBoxRound, kBoxRound));
+                    float h0, h1, l0, l1;
+                    upk(hi, h0, h1);
+                    upk(lo, l0, l1);
+                    int *c = (o[k] < slot0 ? cell : cell0) + o[k];
+                    atomicAdd(c, __float_as_int(h0) - kBoxRoundBits);
+                    atomicAdd(c + 4, __float_as_int(h1) - kBoxRoundBits);
+                    atomicAdd(c + cells, __float_as_int(l0) - kBoxRoundBits);
+                    atomicAdd(c + cells + 4, __float_as_int(l1) - kBoxRoundBits);
+                }
+            } else {
+#pragma unroll 1
+                for (int k = 0; k < 4; ++k) {
+                    const uint32_t pi = __shfl_sync(0xffffffffu, pos, 2 * (i + k));
+                    float *np = a.num[p] + f * a.frame_stride + (long long)(unpack_y(pi) + sy) * a.ld + unpack_x(pi) + sx;
+                    atomicAdd(np, v[(i + k) * 2 * kBT]);
+                    atomicAdd(np + 4, v[(i + k) * 2 * kBT + 32]);
+                }
+            }
+        }
+        if (active && h == 0) atomicAdd(a.wmap[p] + f * a.frame_stride + (long long)unpack_y(pos) * a.ld + unpack_x(pos), denW);
+        __syncwarp();
+    }
+
+    // the box, then the slot of block (0, 0), to the numerator plane
+    __syncthreads();
+    float *num = a.num[p] + f * a.frame_stride;
+    for (int e = threadIdx.x; e < bh * qw; e += NP * 64) {
+        const int yy = e / qw, c = 4 * (e - yy * qw);
+        const int4 hi = *reinterpret_cast<const int4 *>(acc + yy * P + c), lo = *reinterpret_cast<const int4 *>(acc + cells + yy * P + c);
+        float *d = num + (long long)(y0 + yy) * a.ld + x0 + c;
+        if (hi.x | hi.y | hi.z | hi.w | lo.x | lo.y | lo.z | lo.w)
+            atomicAdd(reinterpret_cast<float4 *>(d), make_float4(box_value(hi.x, lo.x), box_value(hi.y, lo.y),
+                                                                 box_value(hi.z, lo.z), box_value(hi.w, lo.w)));
+    }
+    if (threadIdx.x < 64) {
+        const int e = slot0 + threadIdx.x;
+        if (acc[e] | acc[cells + e]) atomicAdd(num + (long long)(threadIdx.x >> 3) * a.ld + (threadIdx.x & 7), box_value(acc[e], acc[cells + e]));
+    }
+}
+
+}  // namespace bm3d

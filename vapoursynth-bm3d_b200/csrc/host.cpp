@@ -263,7 +263,6 @@ static const DeviceTables &device_tables()
     DeviceTables &t = g_dev[dev];
     if (!t.ready) {
         const std::vector<float> odd = host_odd_tables();
-        CU(upload_odd_tables(odd.data()));
         CU(cudaMalloc(&t.odd_all, sizeof(float) * odd.size()));
         CU(cudaMemcpy(t.odd_all, odd.data(), sizeof(float) * odd.size(), cudaMemcpyHostToDevice));
         t.ready = true;
@@ -1280,6 +1279,21 @@ public:
             CU(launch_cf_partial_list(cnt, ngroups, para.G, pl, pn, stream));
             a.plist = pl;
             a.plist_n = pn;
+        }
+        if (fast && !v && !a.plist) {
+            CFBox g{};
+            g.scan_y = d_sy.as<int>();
+            g.scan_x = d_sx.as<int>();
+            g.nby = (int)sy.size();
+            g.nbx = (int)sx.size();
+            g.range = para.R / para.bmstep * para.bmstep;
+            for (int p = 0; p < 3; ++p)
+                if (a.process[p]) g.plane[g.nplanes++] = p;
+            cudaError_t e = cudaSuccess;
+            if (launch_cf_box(a, g, para.step, stream, &e)) {
+                CU(e);
+                return;
+            }
         }
         if (fast) CU(launch_cf_fast(a, stream));
         if (!fast) {

@@ -8,6 +8,7 @@
 #include "proposal.cuh"
 #include "vbm.cuh"
 #include "cf.cuh"
+#include "cf_box.cuh"
 #include "cf_tc.cuh"
 #include "fp64.cuh"
 #include "convert.cuh"
@@ -26,11 +27,6 @@ static std::atomic<unsigned long long> g_launches{0};
 unsigned long long launch_count() { return g_launches.load(); }
 void count_launch() { g_launches.fetch_add(1, std::memory_order_relaxed); }
 #define COUNT_LAUNCH() g_launches.fetch_add(1, std::memory_order_relaxed)
-
-cudaError_t upload_odd_tables(const float *host_odd_all)
-{
-    return cudaMemcpyToSymbol(c_odd, host_odd_all, sizeof(float) * kOddConstFloats);
-}
 
 template <typename K>
 static cudaError_t allow_smem(K kernel, size_t bytes)
@@ -159,21 +155,70 @@ cudaError_t launch_vbm_predict(const VBMArgs &a, bool fast, int nframes, size_t 
 
 int cf_fast_supported(int B, int G) { return B == 8 && (G == 8 || G == 16 || G == 32); }
 
+// Tile of reference blocks for cf_box_kernel with NP warp pairs and at most `cap` bytes of shared memory
+// per CTA (0: none fits); fills the geometry.  A pair takes one slot of 32 / G groups per step, and staging
+// and flushing the box cost about half a step, so the tile with the most groups per (steps + 1/2) is taken.
+static int cf_box_fit(const CFArgs &a, CFBox &g, int step, int G, int NP, size_t cap, size_t *smem)
+{
+    const int gpw = 32 / G;
+    double best = 0.0;
+    for (int ny = 1; ny <= 8; ++ny)
+        for (int nx = gpw; nx * ny <= 128; nx += gpw) {
+            const int w = (2 * g.range + 8 + (nx - 1) * step + 3 + 3) & ~3;
+            const int rows = std::min(a.H, 2 * g.range + 8 + (ny - 1) * step);
+            const int pitch = w + ((12 - (w & 7)) & 7);      // 4 mod 8: a scatter step's eight rows in distinct banks
+            const size_t bytes = (size_t)NP * 32 * kBT * 8 + ((size_t)rows * pitch + 64) * 16 + (size_t)NP * 2 * gpw * 4;
+            if (bytes > cap) break;
+            const int steps = (ny * (nx / gpw) + NP - 1) / NP;
+            const double gain = std::min(nx, g.nbx) * std::min(ny, g.nby) / (steps + 0.5);
+            if (gain <= best) continue;
+            best = gain;
+            g.tx = (g.nbx + nx - 1) / nx;
+            g.ty = (g.nby + ny - 1) / ny;
+            g.rows = rows;
+            g.pitch = pitch;
+            *smem = bytes;
+        }
+    return best > 0.0;
+}
+
+template <int G, int NP>
+static cudaError_t launch_cf_box_t(const CFArgs &a, const CFBox &g, size_t smem, cudaStream_t s)
+{
+    cudaError_t e;
+    if ((e = allow_smem(cf_box_kernel<G, NP>, smem)) != cudaSuccess) return e;
+    const long long frames = a.ngroups / a.blocks_per_frame;
+    COUNT_LAUNCH();
+    cf_box_kernel<G, NP><<<dim3((unsigned)(frames * g.tx * g.ty), g.nplanes), NP * 64, smem, s>>>(a, g);
+    return cudaGetLastError();
+}
+
+template <int G>
+static int launch_cf_box_g(const CFArgs &a, CFBox g, int step, cudaStream_t s, cudaError_t *e)
+{
+    size_t smem = 0;
+    // two CTAs of four pairs per SM; else three of two pairs; else one CTA of four pairs
+    if (cf_box_fit(a, g, step, G, 4, 115712, &smem)) return *e = launch_cf_box_t<G, 4>(a, g, smem, s), 1;
+    if (cf_box_fit(a, g, step, G, 2, 76800, &smem)) return *e = launch_cf_box_t<G, 2>(a, g, smem, s), 1;
+    if (cf_box_fit(a, g, step, G, 4, 232448, &smem)) return *e = launch_cf_box_t<G, 4>(a, g, smem, s), 1;
+    return 0;
+}
+
+int launch_cf_box(const CFArgs &a, const CFBox &g, int step, cudaStream_t s, cudaError_t *e)
+{
+    if (a.B != 8 || !a.wiener || a.vbm3d) return 0;
+    switch (a.G) {
+    case 8: return launch_cf_box_g<8>(a, g, step, s, e);
+    case 16: return launch_cf_box_g<16>(a, g, step, s, e);
+    case 32: return launch_cf_box_g<32>(a, g, step, s, e);
+    default: return 0;
+    }
+}
+
 template <int G, bool W>
 static cudaError_t launch_cf_fast_t(const CFArgs &a, cudaStream_t s)
 {
     cudaError_t e;
-    if constexpr (W) if (!a.skip_full && !a.vbm3d) {
-        // Final over all groups of BM3D frames: runs of consecutive groups, one per CTA
-        const size_t smem = (size_t)kCfWarps * 2 * 32 * kTP * sizeof(float) + kCfCells * sizeof(unsigned long long) +
-                            kCfWarps * 8 * sizeof(int);
-        const long long runs = (a.ngroups + kCfRunGroups - 1) / kCfRunGroups;
-        const int grid = (int)std::max<long long>(1, std::min<long long>(runs, 1LL << 20));
-        if ((e = allow_smem(cf_run_kernel<G, W>, smem)) != cudaSuccess) return e;
-        COUNT_LAUNCH();
-        cf_run_kernel<G, W><<<grid, 32 * kCfWarps, smem, s>>>(a);
-        return cudaGetLastError();
-    }
     // per-lane kernel: 4 warps per CTA, grid-stride over the groups
     const int warps = 4;
     const long long warps_needed = (a.ngroups + (32 / G) - 1) / (32 / G);

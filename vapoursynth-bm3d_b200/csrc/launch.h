@@ -8,9 +8,6 @@
 
 namespace bm3d {
 
-// Copies the odd-part DCT tables for N = 2..64 into constant memory of the current device.
-cudaError_t upload_odd_tables(const float *host_odd_all);
-
 cudaError_t launch_bm_full(const BMArgs &a, int nframes, size_t smem_bytes, cudaStream_t s);
 // Learned proposal (no reference counterpart): feature network forward into bf16 hidden /
 // feature planes [16][H][W] (hid, feat), fp32 row sums rs [16][H][W - 7] and bf16 block descriptors
@@ -35,8 +32,11 @@ cudaError_t launch_bm_tc(const BMArgs &a, const BmtLayout &L, int nframes, cudaS
 // fast: the register-blocked kernel (B = 8, ps_step 1, ps_num <= 2, G <= 32, no descriptors,
 // ps_range <= kPsMaxRange); same lists
 cudaError_t launch_vbm_predict(const VBMArgs &a, bool fast, int nframes, size_t smem_bytes, cudaStream_t s);
+// Plain Final filter of BM3D frames (B = 8, G in {8, 16, 32}) with a run's image region in shared
+// memory; returns 0 if the shape is not its own or the region does not fit, else 1 and the status.
+int launch_cf_box(const CFArgs &a, const CFBox &g, int step, cudaStream_t s, cudaError_t *e);
 // Fast collaborative filter (B = 8, G in {8, 16, 32}, any group length n <= G); sizes its own
-// grid (one CTA per run of consecutive groups); returns cudaErrorInvalidValue for other shapes.
+// grid; returns cudaErrorInvalidValue for other shapes.
 cudaError_t launch_cf_fast(const CFArgs &a, cudaStream_t s);
 // Indices of the groups with count < G into list (device counter n, zeroed by the caller).
 cudaError_t launch_cf_partial_list(const int *count, long long ngroups, int G, long long *list, unsigned int *n, cudaStream_t s);

@@ -63,9 +63,8 @@ long long round64(long long n) { return (n + 63) / 64 * 64; }
 std::mutex g_setup_mutex;
 float *g_dev_scratch[kMaxDevices];       // device address of the array, per device (set-up done)
 
-// Host image of the table region and of the constant odd tables (N = 2..64), built once.
+// Host image of the table region, built once.
 float g_table_image[kTableFloats];
-float g_odd_image[1365];
 bool g_images_ready = false;
 
 void build_images()
@@ -84,13 +83,6 @@ void build_images()
     for (int N = 0; N < kOffFloats; ++N) {
         const int v = N <= kMaxGroup ? off[N] : -1;
         std::memcpy(&g_table_image[N], &v, sizeof(int));
-    }
-    int o = 0;
-    for (int N = 2; N <= 64; N *= 2) {
-        const int h = N / 2;
-        for (int m = 0; m < h; ++m)
-            for (int j = 0; j < h; ++j) g_odd_image[o + m * h + j] = cos2((long)(2 * j + 1) * (2 * m + 1), 2L * N);
-        o += h * h;
     }
     g_images_ready = true;
 }
@@ -113,7 +105,6 @@ int setup_device(int dev, float **out)
     float *ptr = nullptr;
     cudaError_t e = cudaGetSymbolAddress((void **)&ptr, g_noalloc_scratch);
     if (e != cudaSuccess) return set_error(BM3D_ERR_CUDA, cuda_text("cudaGetSymbolAddress", e));
-    if ((e = upload_odd_tables(g_odd_image)) != cudaSuccess) return set_error(BM3D_ERR_CUDA, cuda_text("table upload", e));
     if ((e = cudaMemcpy(ptr, g_table_image, sizeof(g_table_image), cudaMemcpyHostToDevice)) != cudaSuccess)
         return set_error(BM3D_ERR_CUDA, cuda_text("table upload", e));
     g_dev_scratch[dev] = ptr;
