@@ -60,41 +60,29 @@ BM3D_HD inline int vbm8_warp_floats(int range, int sp_cap, int list_cap, int G)
     return (64 + vbm8_work_floats(range, sp_cap, list_cap) + 2 * list_cap + 2 * G + 2 + 3) & ~3;
 }
 
-// Precision-form block matching (bm_tc_kernel): at most kBmtRefs reference blocks per CTA and
-// kBmtCols candidate columns (the union of their search windows along the row).
-constexpr int kBmtRefs = 8;
-constexpr int kBmtCols = 64;
-
-// Shared-memory layout of bm_tc_kernel for a search range (candidate step 1), plane height and
-// reference block step.
-struct BmtLayout {
-    int wh;           // window rows (<= 2 range + 8)
-    int wp;           // window pitch in floats (odd)
-    int nr;           // candidate rows (<= 2 range + 1)
-    int cs;           // per-reference distance slots (>= (2 range + 1)^2 + 1, even)
-    int nrc;          // reference blocks per CTA (their windows span <= kBmtCols columns)
-    int offU, offR, offWin, offRsq, offSd, offScr, bytes;
+// bm_est_kernel: window pitch in row pairs, place of the pairs that start at odd rows, pairs in all,
+// distance slots per reference block, reference blocks on the regular grid of a row and teams of four of them
+struct EstLayout {
+    int pitch, odd, cells, cs, nreg, teams, bytes;
 };
+constexpr int kEstMaxStep = 8;
 
-// nrc = 0: the range is too wide for the form
-inline BmtLayout bmt_layout(int range, int H, int block_step)
+// nbx, last: reference blocks of a row and the position of the last one; W: displacements per lane
+inline EstLayout est_layout(int range, int step, int W, int nbx, int last)
 {
-    BmtLayout L{};
-    const int span = 2 * range + 1;
-    L.nrc = span > kBmtCols ? 0 : (kBmtCols - span) / block_step + 1;
-    if (L.nrc > kBmtRefs) L.nrc = kBmtRefs;
-    L.nr = span < H - 7 ? span : H - 7;
-    L.wh = L.nr + 7;
-    L.wp = (kBmtCols + 7) | 1;
-    L.cs = (span * span + 1 + 1) & ~1;
-    int o = 0;
-    L.offU = o;   o += (L.wh + 1) * kBmtCols * 16;           // fp16 candidate rows (+1 zero row)
-    L.offR = o;   o += 16 * 64 * 2;                          // reference blocks: high terms, low terms
-    L.offWin = o; o += (L.wh * L.wp * 4 + 15) & ~15;         // fp32 window
-    L.offRsq = o; o += L.wh * kBmtCols * 4;                  // row sums of squares of the candidates
-    L.offSd = o;  o += kBmtRefs * L.cs * 4;                  // distance estimates
-    L.offScr = o; o += kBmtRefs * 192 * 4;                   // per-warp selection scratch
-    L.bytes = o;
+    EstLayout L{};
+    const int span = 2 * range + 1, nc = 8 + 3 * step;
+    // lanes on consecutive rows read pairs from even and odd rows in turn: with an odd pitch and the two
+    // sets 8 mod 16 pairs apart, 16 of them fall in distinct banks
+    L.pitch = (3 + 2 * range + nc + W + 3) | 1;        // whole 16-byte chunks
+    L.odd = (range + 4) * L.pitch;
+    L.odd += (24 - L.odd % 16) % 16;
+    L.cells = L.odd + (range + 3) * L.pitch + W;
+    L.cells += L.cells & 1;
+    L.cs = (span * span + 1 + 31) & ~31;
+    L.nreg = last % step ? nbx - 1 : nbx;              // the last block is moved inside the plane
+    L.teams = (L.nreg + 3) / 4;
+    L.bytes = 8 * (4 * ((nc + 1) & ~1) + 32 + L.cells) + 4 * (4 * L.cs + 4 * 320);
     return L;
 }
 

@@ -269,11 +269,11 @@ __device__ __forceinline__ float exact_ssd8_rb(const f32x2 (&rbp)[32], const flo
     return lane_combine(acc);
 }
 
-// Exact SSD (the reference's order) of the 8 x 8 reference block at rp (window, pitch wp) against
+// Exact SSD (the reference's order) of the 8 x 8 reference block at rp (pitch rpitch) against
 // every lattice candidate (rows t + ry s, columns l + c s; window origin wy0, wx0) into
 // sd[ry * ncols + c], and against the trailing (0, 0) candidate of `plane` into sd[nrows * ncols].
 // One warp.
-__device__ __forceinline__ void ssd8_lattice(float *sd, const float *win, int wp, int wy0, int wx0, const float *rp,
+__device__ __forceinline__ void ssd8_lattice(float *sd, const float *win, int wp, int wy0, int wx0, const float *rp, int rpitch,
                                              int t, int l, int s, int nrows, int ncols, const float *plane, long long ld)
 {
     const int lane = (int)lane_id();
@@ -283,7 +283,7 @@ __device__ __forceinline__ void ssd8_lattice(float *sd, const float *win, int wp
 #pragma unroll
     for (int y = 0; y < 8; ++y)
 #pragma unroll
-        for (int m = 0; m < 4; ++m) rbp[y * 4 + m] = pack2(rp[y * wp + 2 * m], rp[y * wp + 2 * m + 1]);
+        for (int m = 0; m < 4; ++m) rbp[y * 4 + m] = pack2(rp[y * rpitch + 2 * m], rp[y * rpitch + 2 * m + 1]);
 
     // item = 4 horizontally adjacent candidates; consecutive lanes take consecutive rows of
     // the same quad column (with the odd window pitch their loads hit distinct banks)
@@ -415,7 +415,7 @@ __global__ void __launch_bounds__(256) bm_full_kernel(BMArgs a)
     const int ctot = clat + 1;
 
     if constexpr (BT == 8) {
-        ssd8_lattice(sd, win, wp, wy0, wx0, win + (j - wy0) * wp + (i - wx0), t, l, s, nrows, ncols, plane, a.ld);
+        ssd8_lattice(sd, win, wp, wy0, wx0, win + (j - wy0) * wp + (i - wx0), wp, t, l, s, nrows, ncols, plane, a.ld);
     } else {
         // generic block size: reference block staged in this warp's shared slice
         float *rblk = hk + 2 * a.G;

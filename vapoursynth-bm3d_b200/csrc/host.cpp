@@ -1165,11 +1165,10 @@ public:
         a.cand_cap = lat * lat + 1;
         a.win_h = std::min(H, 2 * a.range + a.B);
         const bool use_learned = learned_matching();
-        if (tc && !use_learned && para.B == 8 && a.step == 1 && para.G >= 2 && para.G <= 32) {
-            // precision form: distance estimates on the tensor cores, exact lists
-            const BmtLayout L = bmt_layout(a.range, H, para.step);
-            if (L.nrc >= 1 && L.bytes <= 200 * 1024) {
-                CU(launch_bm_tc(a, L, nout, stream));
+        if (!use_learned) {
+            cudaError_t e = cudaSuccess;
+            if (launch_bm_est(a, para.step, sx.back(), nout, stream, &e)) {
+                CU(e);
                 return;
             }
         }

@@ -4,7 +4,7 @@
 #include "common.cuh"
 #include "select.cuh"
 #include "bm.cuh"
-#include "bm_tc.cuh"
+#include "bm_est.cuh"
 #include "proposal.cuh"
 #include "vbm.cuh"
 #include "cf.cuh"
@@ -33,18 +33,6 @@ static cudaError_t allow_smem(K kernel, size_t bytes)
 {
     if (bytes <= 48 * 1024) return cudaSuccess;
     return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-}
-
-cudaError_t launch_bm_tc(const BMArgs &a, const BmtLayout &L, int nframes, cudaStream_t s)
-{
-    dim3 grid((a.nbx + L.nrc - 1) / L.nrc, a.nby, nframes);
-    // at most two CTAs per SM, so that their 256 tensor-memory columns each are never contended
-    const size_t smem = std::max<size_t>((size_t)L.bytes, 76 * 1024);
-    cudaError_t e;
-    if ((e = allow_smem(bm_tc_kernel, smem)) != cudaSuccess) return e;
-    COUNT_LAUNCH();
-    bm_tc_kernel<<<grid, kBmtThreads, smem, s>>>(a, L);
-    return cudaGetLastError();
 }
 
 // ---- learned proposal ----------------------------------------------------------------------------
@@ -117,6 +105,36 @@ cudaError_t launch_bm_learned(const BMArgs &a, const void *desc, int nprop, int 
     COUNT_LAUNCH();
     bm_learned_kernel<<<grid, 32 * a.warps, smem, s>>>(a, static_cast<const __nv_bfloat16 *>(desc), nprop);
     return cudaGetLastError();
+}
+
+template <int S, int W>
+static cudaError_t launch_bm_est_t(const BMArgs &a, const EstLayout &L, int nframes, cudaStream_t s)
+{
+    cudaError_t e;
+    if ((e = allow_smem(bm_est_kernel<S, W>, L.bytes)) != cudaSuccess) return e;
+    COUNT_LAUNCH();
+    bm_est_kernel<S, W><<<dim3(L.teams + (L.nreg < a.nbx), a.nby, nframes), 128, L.bytes, s>>>(a, L);
+    return cudaGetLastError();
+}
+
+int launch_bm_est(const BMArgs &a, int block_step, int last, int nframes, cudaStream_t s, cudaError_t *e)
+{
+    if (a.B != 8 || a.step != 1 || a.G < 2 || a.G > 32 || block_step > kEstMaxStep) return 0;
+    // displacements per lane: 3 or 4, whichever leaves fewer slots of the team's 128 lanes unused
+    const int span = 2 * a.range + 1;
+    if (span * span >= 1 << 15) return 0;
+    auto slots = [span](int W) { return ((span + W - 1) / W * span + 127) / 128 * W; };
+    const int W = slots(4) < slots(3) ? 4 : 3;
+    const EstLayout L = est_layout(a.range, block_step, W, a.nbx, last);
+    if (L.bytes > 200 * 1024) return 0;
+    switch (block_step * 8 + W) {
+#define BM3D_EST(S) \
+    case S * 8 + 3: *e = launch_bm_est_t<S, 3>(a, L, nframes, s); return 1; \
+    case S * 8 + 4: *e = launch_bm_est_t<S, 4>(a, L, nframes, s); return 1;
+    BM3D_EST(1) BM3D_EST(2) BM3D_EST(3) BM3D_EST(4) BM3D_EST(5) BM3D_EST(6) BM3D_EST(7) BM3D_EST(8)
+#undef BM3D_EST
+    default: return 0;
+    }
 }
 
 cudaError_t launch_bm_full(const BMArgs &a, int nframes, size_t smem, cudaStream_t s)
