@@ -1,4 +1,4 @@
-"""Plain Final filter with the image region of a tile in shared memory, against the oracle: tile and
+"""Plain Basic and Final filters with the image region of a tile in shared memory, against the oracle: tile and
 slot edges, every kind of group length, block (0, 0) inside and outside the box, terms too large for
 the fixed-point box, NaN, and search ranges at and beyond the largest box.
 
@@ -23,8 +23,13 @@ def pair(h, w, sigma=10.0, seed=3):
 
 
 def check(orc, src, ref, profile="np", **over):
-    got = core.bm3d.Final(source(src, "GRAY"), source(ref, "GRAY"), profile=profile, matrix=6, **over).numpy()
-    p = orc.default_params(1, False, profile, 10.0, matrix=6, **over)
+    """ref None: Basic of src"""
+    if ref is None:
+        node = core.bm3d.Basic(source(src, "GRAY"), profile=profile, matrix=6, **over)
+    else:
+        node = core.bm3d.Final(source(src, "GRAY"), source(ref, "GRAY"), profile=profile, matrix=6, **over)
+    got = node.numpy()
+    p = orc.default_params(0 if ref is None else 1, False, profile, 10.0, matrix=6, **over)
     exp = orc.bm3d(p, src, ref, threads=8)
     assert np.array_equal(np.isnan(got), np.isnan(exp))
     ok = ~np.isnan(exp)
@@ -32,7 +37,7 @@ def check(orc, src, ref, profile="np", **over):
     assert np.abs(got - exp)[ok].max() <= REL * scale
 
 
-@pytest.mark.parametrize("h,w,over", [
+CASES = [
     (8, 8, {}),                                                  # one block: one group of one
     (9, 47, {}),                                                 # window taller than the frame
     (41, 13, {}),                                                # window wider than the frame
@@ -47,9 +52,20 @@ def check(orc, src, ref, profile="np", **over):
     (120, 140, {"bm_range": 36}),                                # one CTA per SM
     (200, 230, {"bm_range": 60, "block_step": 8}),               # beyond any box: per-lane kernel
     (64, 80, {"bm_range": 6, "bm_step": 4}),                     # range rounded down to the step
-])
+]
+
+
+@pytest.mark.parametrize("h,w,over", CASES)
 def test_final_matches_oracle(orc, h, w, over):
     check(orc, *pair(h, w), **over)
+
+
+@pytest.mark.parametrize("h,w,over", CASES)
+def test_basic_matches_oracle(orc, h, w, over):
+    """Two slots at a time: odd numbers of slots and of groups in them, and groups of different lengths."""
+    if "th_mse" in over:
+        over = dict(over, th_mse=300.0)                          # noisy blocks: short groups below it
+    check(orc, pair(h, w)[0], None, **over)
 
 
 def test_block_at_origin_in_distant_groups(orc):
@@ -64,9 +80,11 @@ def test_block_at_origin_in_distant_groups(orc):
 def test_terms_beyond_the_fixed_point_box(orc):
     src, ref = pair(56, 72)
     check(orc, src * np.float32(1e6), ref * np.float32(1e6), th_mse=1e15)
+    check(orc, src * np.float32(1e6), None, th_mse=1e15)
 
 
 def test_nan_stays_in_the_groups_that_hold_it(orc):
     src, ref = pair(64, 96)
     src[0, 0, 30, 40] = np.nan
     check(orc, src, ref, th_mse=40.0)
+    check(orc, src, None)

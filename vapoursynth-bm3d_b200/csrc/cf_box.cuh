@@ -199,18 +199,17 @@ __device__ __forceinline__ f2 shfl_pair(f2 v)
     return pk(__shfl_xor_sync(0xffffffffu, a, 1), __shfl_xor_sync(0xffffffffu, b, 1));
 }
 
-// Block at `b` (pitch P cells) of the box of (reference, source) pairs -> its 2-D coefficients at `t`.
-// Lane half h (lane & 1) transforms rows 0 .. 3 (h = 0) or 7 .. 4 (h = 1), then the columns 2k + h.
-__device__ __forceinline__ void box_forward(const f2 *b, int P, f2 *t, int h)
+// A block's pixels, load(y, x) -> its 2-D coefficients at `t`.  Lane half h (lane & 1) transforms rows 0 .. 3
+// (h = 0) or 7 .. 4 (h = 1), then the columns 2k + h; load(i, x) gives pixel x of the lane's i-th row.
+template <class Load>
+__device__ __forceinline__ void box_forward(Load &&load, f2 *t, int h)
 {
     f2 keep[4][4], give[4][4];            // [row][column pair]: columns 2k + h, columns 2k + 1 - h
-    const int step = h ? -P : P;
-    b += h ? 7 * P : 0;
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
         f2 x[8], X[8];
 #pragma unroll
-        for (int k = 0; k < 8; ++k) x[k] = b[i * step + k];
+        for (int k = 0; k < 8; ++k) x[k] = load(i, k);
         fdct2<8>(x, [&](int k, int st, const auto &v) {
 #pragma unroll
             for (int c = 0; c < (int)(sizeof(v) / sizeof(v[0])); ++c) X[k + c * st] = v[c];
@@ -292,6 +291,21 @@ __device__ __forceinline__ void box_inverse(float *t, float scale, bool active, 
     }
 }
 
+// adds the halves of v to the cells at c0 and c1 (high words; the low words are `low` further on)
+__device__ __forceinline__ void box_add(f2 v, int *c0, int *c1, int low)
+{
+    const f2 hi = fma2(v, pk(kBoxHi, kBoxHi), pk(kBoxRound, kBoxRound));
+    const f2 rest = fma2(sub2(hi, pk(kBoxRound, kBoxRound)), pk(-kBoxHiUnit, -kBoxHiUnit), v);
+    const f2 lo = fma2(rest, pk(kBoxLo, kBoxLo), pk(kBoxRound, kBoxRound));
+    float h0, h1, l0, l1;
+    upk(hi, h0, h1);
+    upk(lo, l0, l1);
+    atomicAdd(c0, __float_as_int(h0) - kBoxRoundBits);
+    atomicAdd(c1, __float_as_int(h1) - kBoxRoundBits);
+    atomicAdd(c0 + low, __float_as_int(l0) - kBoxRoundBits);
+    atomicAdd(c1 + low, __float_as_int(l1) - kBoxRoundBits);
+}
+
 // Wiener z stage of one coefficient column (cells t[z * kBT]) of a group of N blocks: the filtered source
 // column into the cells' low words; returns the sum of the squared weights
 template <int N>
@@ -353,6 +367,24 @@ __device__ __forceinline__ float box_wiener_any(int at, float sg, int n, const C
     if (n == 2) return box_wiener<2>(at, sg);
     if (n == 1) return box_wiener<1>(at, sg);
     return box_wiener_direct(at, sg, n, dtab_for(a, n, false), dtab_for(a, n, true));
+}
+
+// the box, then the slot of block (0, 0), to the numerator plane
+__device__ __forceinline__ void box_flush(const int *acc, int cells, int slot0, int P, float *num, int ld, int y0, int x0, int bh, int bw)
+{
+    const int qw = bw >> 2;
+    for (int e = threadIdx.x; e < bh * qw; e += blockDim.x) {
+        const int yy = e / qw, c = 4 * (e - yy * qw);
+        const int4 hi = *reinterpret_cast<const int4 *>(acc + yy * P + c), lo = *reinterpret_cast<const int4 *>(acc + cells + yy * P + c);
+        float *d = num + (long long)(y0 + yy) * ld + x0 + c;
+        if (hi.x | hi.y | hi.z | hi.w | lo.x | lo.y | lo.z | lo.w)
+            atomicAdd(reinterpret_cast<float4 *>(d), make_float4(box_value(hi.x, lo.x), box_value(hi.y, lo.y),
+                                                                 box_value(hi.z, lo.z), box_value(hi.w, lo.w)));
+    }
+    if (threadIdx.x < 64) {
+        const int e = slot0 + threadIdx.x;
+        if (acc[e] | acc[cells + e]) atomicAdd(num + (long long)(threadIdx.x >> 3) * ld + (threadIdx.x & 7), box_value(acc[e], acc[cells + e]));
+    }
 }
 
 template <int G, int NP>
@@ -442,7 +474,10 @@ __global__ void __launch_bounds__(NP * 64, 8 / NP) cf_box_kernel(CFArgs a, CFBox
         const int off = !active ? 0 : in ? (y - y0) * P + x - x0 : slot0;
         const uint32_t pos = active ? pos1 : 0u;
         fetch(slot + NP, n1, pos1);
-        box_forward(box + off, off < slot0 ? P : 8, tb, h);
+        const int bp = off < slot0 ? P : 8;
+        const f2 *b = box + off + (h ? 7 * bp : 0);
+        const int step = h ? -bp : bp;
+        box_forward([&](int i, int c) { return b[i * step + c]; }, tb, h);
         pair_barrier(1 + pair);
         // z stage: warp `role` takes columns 32 role .. 32 role + 31 of every group of the slot
         int sbx;
@@ -480,17 +515,8 @@ __global__ void __launch_bounds__(NP * 64, 8 / NP) cf_box_kernel(CFArgs a, CFBox
             if (__all_sync(0xffffffffu, fits)) {
 #pragma unroll
                 for (int k = 0; k < 4; ++k) {
-                    const f2 hi = fma2(e[k], pk(kBoxHi, kBoxHi), pk(kBoxRound, kBoxRound));
-                    const f2 rest = fma2(sub2(hi, pk(kBoxRound, kBoxRound)), pk(-kBoxHiUnit, -kBoxHiUnit), e[k]);
-                    const f2 lo = fma2(rest, pk(kBoxLo, kBoxLo), pk(kBoxRound, kBoxRound));
-                    float h0, h1, l0, l1;
-                    upk(hi, h0, h1);
-                    upk(lo, l0, l1);
                     int *c = (o[k] < slot0 ? cell : cell0) + o[k];
-                    atomicAdd(c, __float_as_int(h0) - kBoxRoundBits);
-                    atomicAdd(c + 4, __float_as_int(h1) - kBoxRoundBits);
-                    atomicAdd(c + cells, __float_as_int(l0) - kBoxRoundBits);
-                    atomicAdd(c + cells + 4, __float_as_int(l1) - kBoxRoundBits);
+                    box_add(e[k], c, c + 4, cells);
                 }
             } else {
 #pragma unroll 1
@@ -506,21 +532,301 @@ __global__ void __launch_bounds__(NP * 64, 8 / NP) cf_box_kernel(CFArgs a, CFBox
         __syncwarp();
     }
 
-    // the box, then the slot of block (0, 0), to the numerator plane
     __syncthreads();
-    float *num = a.num[p] + f * a.frame_stride;
-    for (int e = threadIdx.x; e < bh * qw; e += NP * 64) {
-        const int yy = e / qw, c = 4 * (e - yy * qw);
-        const int4 hi = *reinterpret_cast<const int4 *>(acc + yy * P + c), lo = *reinterpret_cast<const int4 *>(acc + cells + yy * P + c);
-        float *d = num + (long long)(y0 + yy) * a.ld + x0 + c;
-        if (hi.x | hi.y | hi.z | hi.w | lo.x | lo.y | lo.z | lo.w)
-            atomicAdd(reinterpret_cast<float4 *>(d), make_float4(box_value(hi.x, lo.x), box_value(hi.y, lo.y),
-                                                                 box_value(hi.z, lo.z), box_value(hi.w, lo.w)));
+    box_flush(acc, cells, slot0, P, a.num[p] + f * a.frame_stride, a.ld, y0, x0, bh, bw);
+}
+
+// ---- Basic: hard threshold ------------------------------------------------------------------------------
+// A pair of warps takes two slots at once, packed: the halves of every cell and register are the blocks at
+// the same place of slots A and B, through both directions of the transform.
+// Bound: the shared-memory pipe (random-row loads of the blocks, transposes, and four native atomics a
+// pixel pair: 6.7 k of a step's 25 k clocks are atomics).  1920x1080 RGB x 8, step 4, G = 16: 12.6 ms with
+// per-lane gathers and float atomics on the plane (cf_fast_kernel), 8.3 ms now.
+
+// hard threshold of both halves of x, counted in the halves of kept
+__device__ __forceinline__ f2 keep2(f2 x, float ta, float tb, int &kept)
+{
+    float a, b;
+    upk(x, a, b);
+    const bool ka = fabsf(a) > ta, kb = fabsf(b) > tb;
+    kept += (ka ? 1 : 0) + (kb ? 1 << 16 : 0);
+    return pk(ka ? a : 0.0f, kb ? b : 0.0f);
+}
+
+// z stage of one coefficient column of two groups of N blocks; thresholds t0 (z = 0) and t1; returns the
+// kept counts in the halves of an int
+template <int N>
+__device__ __noinline__ int box_hard(int at, float t0, float t1)
+{
+    extern __shared__ __align__(16) float smem[];
+    f2 *t = reinterpret_cast<f2 *>(smem) + at;
+    f2 x[N], X[N], y[N];
+#pragma unroll
+    for (int z = 0; z < N; ++z) x[z] = t[z * kBT];
+    int kept = 0;
+    fdct2<N>(x, [&](int k, int st, const auto &v) {
+#pragma unroll
+        for (int i = 0; i < (int)(sizeof(v) / sizeof(v[0])); ++i) {
+            const float th = k + i * st == 0 ? t0 : t1;
+            X[k + i * st] = keep2(v[i], th, th, kept);
+        }
+    });
+    if constexpr (N == 1) y[0] = X[0];
+    else idct2<N>(X, y);
+#pragma unroll
+    for (int z = 0; z < N; ++z) t[z * kBT] = y[z];
+    return kept;
+}
+
+// the same for one of the two groups alone (t: its half of the column), any length
+template <int N>
+__device__ __forceinline__ int box_hard_half(float *t, float t0, float t1)
+{
+    float x[N], X[N];
+#pragma unroll
+    for (int z = 0; z < N; ++z) x[z] = t[2 * z * kBT];
+    fdct_reg<N>(x, X);
+    int kept = 0;
+#pragma unroll
+    for (int z = 0; z < N; ++z) {
+        const bool k = fabsf(X[z]) > (z ? t1 : t0);
+        kept += k;
+        X[z] = k ? X[z] : 0.0f;
     }
-    if (threadIdx.x < 64) {
-        const int e = slot0 + threadIdx.x;
-        if (acc[e] | acc[cells + e]) atomicAdd(num + (long long)(threadIdx.x >> 3) * a.ld + (threadIdx.x & 7), box_value(acc[e], acc[cells + e]));
+    idct_reg<N>(X, x);
+#pragma unroll
+    for (int z = 0; z < N; ++z) t[2 * z * kBT] = x[z];
+    return kept;
+}
+
+__device__ __noinline__ int box_hard_any(int at, int half, float t0, float t1, int n, const float *fwd, const float *inv)
+{
+    extern __shared__ __align__(16) float smem[];
+    float *t = smem + 2 * at + half;
+    switch (n) {
+    case 0: return 0;
+    case 1: return box_hard_half<1>(t, t0, t1);
+    case 2: return box_hard_half<2>(t, t0, t1);
+    case 4: return box_hard_half<4>(t, t0, t1);
+    case 8: return box_hard_half<8>(t, t0, t1);
+    case 16: return box_hard_half<16>(t, t0, t1);
+    case 32: return box_hard_half<32>(t, t0, t1);
     }
+    float X[32], Y[32];
+    direct_sums2<2 * kBT>(t, t, fwd, n, true, X, Y);
+    int kept = 0;
+    for (int z = 0; z < n; ++z) {
+        const bool k = fabsf(X[z]) > (z ? t1 : t0);
+        kept += k;
+        t[2 * z * kBT] = k ? X[z] : 0.0f;
+    }
+    direct_sums2<2 * kBT>(t, t, inv, n, false, X, Y);
+    for (int z = 0; z < n; ++z) t[2 * z * kBT] = X[z];
+    return kept;
+}
+
+// Inverse 2-D transform of both halves of the cells at `t`, scaled, in place: pixel (y, x) to cell 8 x + y.
+// Lane half h inverts the columns 2k + h, then the rows 2i + h.
+__device__ __forceinline__ void box_inverse2(f2 *t, f2 scale, bool activeA, bool activeB, int h)
+{
+    f2 keep[4][4], give[4][4];            // [row][column]
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        f2 X[8], y[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) X[i] = t[i * 8 + 2 * k + h];
+        idct2<8>(X, y);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            keep[i][k] = h ? y[2 * i + 1] : y[2 * i];
+            give[i][k] = h ? y[2 * i] : y[2 * i + 1];
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int k = 0; k < 4; ++k) give[i][k] = shfl_pair(give[i][k]);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        f2 X[8], y[8];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            X[2 * k] = h ? give[i][k] : keep[i][k];
+            X[2 * k + 1] = h ? keep[i][k] : give[i][k];
+        }
+        idct2<8>(X, y);
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+            float a, b;
+            upk(tc::mul2(y[k], scale), a, b);
+            t[k * 8 + 2 * i + h] = pk(activeA ? a : 0.0f, activeB ? b : 0.0f);
+        }
+    }
+}
+
+template <int G, int NP>
+__global__ void __launch_bounds__(NP * 64, 8 / NP) cf_boxh_kernel(CFArgs a, CFBox g)
+{
+    extern __shared__ __align__(16) float smem[];
+    constexpr int GPW = 32 / G;                     // groups per slot
+    constexpr int kT = 32 * kBT;                    // cells of a transpose buffer
+    const int lane = (int)lane_id();
+    const int warp = threadIdx.x >> 5, pair = warp >> 1, role = warp & 1;
+    const int p = g.plane[blockIdx.y];
+    const int rx = blockIdx.x % g.tx, rest = blockIdx.x / g.tx;
+    const int rr = rest % g.ty, f = rest / g.ty;
+    const int bx0 = (int)((long long)rx * g.nbx / g.tx), bx1 = (int)((long long)(rx + 1) * g.nbx / g.tx);
+    const int by0 = (int)((long long)rr * g.nby / g.ty), by1 = (int)((long long)(rr + 1) * g.nby / g.ty);
+    const int P = g.pitch;
+    const int y0 = max(0, g.scan_y[by0] - g.range), bh = min(a.H, g.scan_y[by1 - 1] + g.range + 8) - y0;
+    const int x0 = max(0, g.scan_x[bx0] - g.range) & ~3;
+    const int bw = (min(a.W, g.scan_x[bx1 - 1] + g.range + 8) - x0 + 3) & ~3;
+    const int slot0 = g.rows * P, cells = slot0 + 64;
+    f2 *tr = reinterpret_cast<f2 *>(smem);
+    int *acc = reinterpret_cast<int *>(tr + NP * kT);                  // high words, then low words
+    float *box = reinterpret_cast<float *>(acc + 2 * cells);
+    int *red = reinterpret_cast<int *>(box + cells) + pair * 2 * GPW;  // [group of the slots][warp]
+    const float *src = a.src[p] + f * a.frame_stride;
+    const int h = lane & 1;
+    const int blk = 16 * role + (lane >> 1);        // the lane's block of a slot: group sub, place z
+    const int sub = blk / G, z = blk - sub * G;
+    const int spr = (bx1 - bx0 + GPW - 1) / GPW, nslots = spr * (by1 - by0);
+    // first group of a slot, and how many groups it has
+    auto slot_at = [&](int slot, int &groups) -> long long {
+        const int sr = slot / spr, bx = bx0 + (slot - sr * spr) * GPW;
+        groups = slot < nslots ? min(GPW, bx1 - bx) : 0;
+        return ((long long)f * g.nby + by0 + sr) * g.nbx + bx;
+    };
+    auto fetch = [&](int slot, int &n, uint32_t &pos) {
+        int groups;
+        const long long grp = slot_at(slot, groups) + sub;
+        n = 0;
+        if (sub < groups) {
+            n = a.count[grp];
+            pos = a.pos[grp * G + z];
+        }
+    };
+    int nA = 0, nB = 0;
+    uint32_t pA = 0, pB = 0;
+    fetch(2 * pair, nA, pA);
+    fetch(2 * pair + 1, nB, pB);
+    const int qw = bw >> 2, chunks = bh * qw + 16;
+    for (int e = threadIdx.x; e < chunks; e += NP * 64) {
+        const int yy = e / qw, c = 4 * (e - yy * qw), m = e - (chunks - 16);
+        if (m < 0) tc::cp_async16(box + yy * P + c, src + (long long)(y0 + yy) * a.ld + x0 + c);
+        else tc::cp_async16(box + slot0 + 4 * m, src + (long long)(m >> 1) * a.ld + 4 * (m & 1));
+    }
+    for (int e = threadIdx.x; e < (cells >> 1); e += NP * 64) reinterpret_cast<int4 *>(acc)[e] = make_int4(0, 0, 0, 0);
+    tc::cp_async_wait_all();
+    __syncthreads();
+
+    f2 *tb = tr + pair * kT + blk * kBT;
+    const int sy = lane & 7, sx = lane >> 3;        // the lane's pixel of a block in the scatter (and column sx + 4)
+    auto place = [&](int n, uint32_t pos) {
+        const int y = unpack_y(pos), x = unpack_x(pos);
+        const bool in = y >= y0 && y + 8 <= y0 + bh && x >= x0 && x + 8 <= x0 + bw;
+        return z >= n ? 0 : in ? (y - y0) * P + x - x0 : slot0;
+    };
+    for (int slot = 2 * pair; slot < nslots; slot += 2 * NP) {
+        const int na = min(nA, G), nb = min(nB, G);
+        const bool actA = z < na, actB = z < nb;
+        const uint32_t posA = actA ? pA : 0u, posB = actB ? pB : 0u;
+        const int offA = place(na, posA), offB = place(nb, posB);
+        fetch(slot + 2 * NP, nA, pA);
+        fetch(slot + 2 * NP + 1, nB, pB);
+        {
+            const int ba = offA < slot0 ? P : 8, bb = offB < slot0 ? P : 8;
+            const float *ca = box + offA + (h ? 7 * ba : 0), *cb = box + offB + (h ? 7 * bb : 0);
+            const int sa = h ? -ba : ba, sb = h ? -bb : bb;
+            box_forward([&](int i, int c) { return pk(ca[i * sa + c], cb[i * sb + c]); }, tb, h);
+        }
+        pair_barrier(1 + pair);
+        int gA, gB;
+        const long long grpA = slot_at(slot, gA), grpB = slot_at(slot + 1, gB);
+        const int col = role * 32 + lane, fxy = ((col & 7) == 0) + ((col >> 3) == 0);
+#pragma unroll 1
+        for (int q = 0; q < GPW; ++q) {
+            const int ma = q < gA ? min(a.count[grpA + q], G) : 0, mb = q < gB ? min(a.count[grpB + q], G) : 0;
+            const int at = pair * kT + q * G * kBT + col;
+            int kept;
+            // groups of the same full length together, others one by one
+            if (ma == G && mb == G) kept = box_hard<G>(at, a.thr4[p][G - 1][fxy + 1], a.thr4[p][G - 1][fxy]);
+            else {
+                kept = 0;
+#pragma unroll 1
+                for (int half = 0; half < 2; ++half) {
+                    const int m = half ? mb : ma, i = max(m, 1) - 1;
+                    kept += box_hard_any(at, half, a.thr4[p][i][fxy + 1], a.thr4[p][i][fxy], m, dtab_for(a, m, false),
+                                         dtab_for(a, m, true)) << (16 * half);
+                }
+            }
+            kept = __reduce_add_sync(0xffffffffu, kept);
+            if (lane == 0) red[2 * q + role] = kept;
+        }
+        pair_barrier(1 + pair);
+        const int kept = red[2 * sub] + red[2 * sub + 1], kA = kept & 0xffff, kB = kept >> 16;
+        if (a.retained && z == 0 && h == 0) {
+            if (sub < gA) a.retained[(long long)p * a.ngroups + grpA + sub] = kA;
+            if (sub < gB) a.retained[(long long)p * a.ngroups + grpB + sub] = kB;
+        }
+        const float dA = kA < 1 ? 1.0f : __fdiv_rn(1.0f, (float)kA), dB = kB < 1 ? 1.0f : __fdiv_rn(1.0f, (float)kB);
+        box_inverse2(tb, pk(actA ? __fdiv_rn(dA, a.amp[na - 1]) : 0.0f, actB ? __fdiv_rn(dB, a.amp[nb - 1]) : 0.0f), actA, actB, h);
+        __syncwarp();
+        // aggregation, four blocks (two places of both slots) per step
+        const f2 *v = tr + pair * kT + 16 * role * kBT + lane;
+        int *cell = acc + sy * P + sx, *cell0 = acc + sy * 8 + sx;
+#pragma unroll
+        for (int i = 0; i < 16; i += 2) {
+            f2 e[4];
+            int oa[2], ob[2];
+            bool fits = true;
+#pragma unroll
+            for (int k = 0; k < 2; ++k) {
+                oa[k] = __shfl_sync(0xffffffffu, offA, 2 * (i + k));
+                ob[k] = __shfl_sync(0xffffffffu, offB, 2 * (i + k));
+                e[2 * k] = v[(i + k) * kBT];
+                e[2 * k + 1] = v[(i + k) * kBT + 32];
+            }
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                float u, w;
+                upk(e[k], u, w);
+                fits = fits && fabsf(u) < kBoxMax && fabsf(w) < kBoxMax;
+            }
+            if (__all_sync(0xffffffffu, fits)) {
+#pragma unroll
+                for (int k = 0; k < 2; ++k) {
+                    int *ca = (oa[k] < slot0 ? cell : cell0) + oa[k], *cb = (ob[k] < slot0 ? cell : cell0) + ob[k];
+                    box_add(e[2 * k], ca, cb, cells);
+                    box_add(e[2 * k + 1], ca + 4, cb + 4, cells);
+                }
+            } else {
+#pragma unroll 1
+                for (int k = 0; k < 2; ++k) {
+                    const uint32_t qa = __shfl_sync(0xffffffffu, posA, 2 * (i + k)), qb = __shfl_sync(0xffffffffu, posB, 2 * (i + k));
+                    float *num = a.num[p] + f * a.frame_stride;
+                    float *na_ = num + (long long)(unpack_y(qa) + sy) * a.ld + unpack_x(qa) + sx;
+                    float *nb_ = num + (long long)(unpack_y(qb) + sy) * a.ld + unpack_x(qb) + sx;
+                    float u, w;
+                    upk(v[(i + k) * kBT], u, w);
+                    atomicAdd(na_, u);
+                    atomicAdd(nb_, w);
+                    upk(v[(i + k) * kBT + 32], u, w);
+                    atomicAdd(na_ + 4, u);
+                    atomicAdd(nb_ + 4, w);
+                }
+            }
+        }
+        if (h == 0) {
+            float *wm = a.wmap[p] + f * a.frame_stride;
+            if (actA) atomicAdd(wm + (long long)unpack_y(posA) * a.ld + unpack_x(posA), dA);
+            if (actB) atomicAdd(wm + (long long)unpack_y(posB) * a.ld + unpack_x(posB), dB);
+        }
+        __syncwarp();
+    }
+
+    __syncthreads();
+    box_flush(acc, cells, slot0, P, a.num[p] + f * a.frame_stride, a.ld, y0, x0, bh, bw);
 }
 
 }  // namespace bm3d

@@ -17,6 +17,7 @@
 
 #include <algorithm>
 #include <atomic>
+#include <cmath>
 #include <cstring>
 #include <vector>
 
@@ -173,26 +174,32 @@ cudaError_t launch_vbm_predict(const VBMArgs &a, bool fast, int nframes, size_t 
 
 int cf_fast_supported(int B, int G) { return B == 8 && (G == 8 || G == 16 || G == 32); }
 
-// Tile of reference blocks for cf_box_kernel with NP warp pairs and at most `cap` bytes of shared memory
-// per CTA (0: none fits); fills the geometry.  A pair takes one slot of 32 / G groups per step, and staging
-// and flushing the box cost about half a step, so the tile with the most groups per (steps + 1/2) is taken.
-static int cf_box_fit(const CFArgs &a, CFBox &g, int step, int G, int NP, size_t cap, size_t *smem)
+// Tile of reference blocks for cf_box_kernel / cf_boxh_kernel with NP warp pairs and at most `cap` bytes of shared memory
+// per CTA (0: none fits); fills the geometry.  A pair takes one slot of 32 / G groups per step (Basic: two), and staging
+// and flushing the box cost about half a step: the tile with the least waves x (steps + 1/2) is taken, where
+// `resident` CTAs run at once (so that a small frame gets small tiles and all SMs; 352x288 at profile fast,
+// 1,584 groups: 34 us with the largest tile, 30 us).
+static int cf_box_fit(const CFArgs &a, CFBox &g, int step, int G, int NP, int resident, size_t cap, size_t *smem)
 {
     const int gpw = 32 / G;
+    const int cell = a.wiener ? 16 : 12, per_step = a.wiener ? NP : 2 * NP;   // bytes of a cell, slots of a step
     double best = 0.0;
     for (int ny = 1; ny <= 8; ++ny)
         for (int nx = gpw; nx * ny <= 128; nx += gpw) {
             const int w = (2 * g.range + 8 + (nx - 1) * step + 3 + 3) & ~3;
             const int rows = std::min(a.H, 2 * g.range + 8 + (ny - 1) * step);
             const int pitch = w + ((12 - (w & 7)) & 7);      // 4 mod 8: a scatter step's eight rows in distinct banks
-            const size_t bytes = (size_t)NP * 32 * kBT * 8 + ((size_t)rows * pitch + 64) * 16 + (size_t)NP * 2 * gpw * 4;
+            const size_t bytes = (size_t)NP * 32 * kBT * 8 + ((size_t)rows * pitch + 64) * cell + (size_t)NP * 2 * gpw * 4;
             if (bytes > cap) break;
-            const int steps = (ny * (nx / gpw) + NP - 1) / NP;
-            const double gain = std::min(nx, g.nbx) * std::min(ny, g.nby) / (steps + 0.5);
-            if (gain <= best) continue;
-            best = gain;
-            g.tx = (g.nbx + nx - 1) / nx;
-            g.ty = (g.nby + ny - 1) / ny;
+            const int steps = (ny * (nx / gpw) + per_step - 1) / per_step;
+            const int tx = (g.nbx + nx - 1) / nx, ty = (g.nby + ny - 1) / ny;
+            double waves = (double)tx * ty * g.nplanes * (double)(a.ngroups / a.blocks_per_frame) / resident;
+            if (waves < 6.0) waves = std::ceil(waves);
+            const double cost = waves * (steps + 0.5);
+            if (best > 0.0 && cost >= best) continue;
+            best = cost;
+            g.tx = tx;
+            g.ty = ty;
             g.rows = rows;
             g.pitch = pitch;
             *smem = bytes;
@@ -203,11 +210,12 @@ static int cf_box_fit(const CFArgs &a, CFBox &g, int step, int G, int NP, size_t
 template <int G, int NP>
 static cudaError_t launch_cf_box_t(const CFArgs &a, const CFBox &g, size_t smem, cudaStream_t s)
 {
+    auto kernel = a.wiener ? cf_box_kernel<G, NP> : cf_boxh_kernel<G, NP>;
     cudaError_t e;
-    if ((e = allow_smem(cf_box_kernel<G, NP>, smem)) != cudaSuccess) return e;
+    if ((e = allow_smem(kernel, smem)) != cudaSuccess) return e;
     const long long frames = a.ngroups / a.blocks_per_frame;
     COUNT_LAUNCH();
-    cf_box_kernel<G, NP><<<dim3((unsigned)(frames * g.tx * g.ty), g.nplanes), NP * 64, smem, s>>>(a, g);
+    kernel<<<dim3((unsigned)(frames * g.tx * g.ty), g.nplanes), NP * 64, smem, s>>>(a, g);
     return cudaGetLastError();
 }
 
@@ -215,16 +223,17 @@ template <int G>
 static int launch_cf_box_g(const CFArgs &a, CFBox g, int step, cudaStream_t s, cudaError_t *e)
 {
     size_t smem = 0;
+    constexpr int sms = 148;
     // two CTAs of four pairs per SM; else three of two pairs; else one CTA of four pairs
-    if (cf_box_fit(a, g, step, G, 4, 115712, &smem)) return *e = launch_cf_box_t<G, 4>(a, g, smem, s), 1;
-    if (cf_box_fit(a, g, step, G, 2, 76800, &smem)) return *e = launch_cf_box_t<G, 2>(a, g, smem, s), 1;
-    if (cf_box_fit(a, g, step, G, 4, 232448, &smem)) return *e = launch_cf_box_t<G, 4>(a, g, smem, s), 1;
+    if (cf_box_fit(a, g, step, G, 4, 2 * sms, 115712, &smem)) return *e = launch_cf_box_t<G, 4>(a, g, smem, s), 1;
+    if (cf_box_fit(a, g, step, G, 2, 3 * sms, 76800, &smem)) return *e = launch_cf_box_t<G, 2>(a, g, smem, s), 1;
+    if (cf_box_fit(a, g, step, G, 4, sms, 232448, &smem)) return *e = launch_cf_box_t<G, 4>(a, g, smem, s), 1;
     return 0;
 }
 
 int launch_cf_box(const CFArgs &a, const CFBox &g, int step, cudaStream_t s, cudaError_t *e)
 {
-    if (a.B != 8 || !a.wiener || a.vbm3d) return 0;
+    if (a.B != 8 || a.vbm3d) return 0;
     switch (a.G) {
     case 8: return launch_cf_box_g<8>(a, g, step, s, e);
     case 16: return launch_cf_box_g<16>(a, g, step, s, e);
