@@ -1182,6 +1182,7 @@ public:
             smem = sizeof(float) * ((size_t)a.win_h * a.win_pitch + (size_t)warps * bm_warp_floats(a.cand_cap, a.G, a.B, a.B != 8));
             if (smem <= 200 * 1024) break;
         }
+        if (a.B != 8) smem += sizeof(float) * (a.B * a.B + 16);    // block (0, 0)
         if (warps < 1) throw std::runtime_error(err("bm_range / block_size too large for the shared-memory search window"));
         if (use_learned) {
             // learned proposals: descriptors of every block position, then the best
@@ -1295,8 +1296,13 @@ public:
             }
         }
         if (fast) CU(launch_cf_fast(a, stream));
+        cudaError_t mid = cudaSuccess;
+        if (!fast && launch_cf_mid(a, stream, &mid)) {
+            CU(mid);
+            return;
+        }
         if (!fast) {
-            // generic path: block sizes other than 8 and group sizes outside {8, 16, 32}; one warp
+            // generic path: blocks beyond 16 x 16 and groups beyond 32 that are not the fast kernels'; one warp
             // per group with a global scratch slot per resident warp (at most 1 GiB in total)
             const long long slot_floats = (long long)para.G * para.B * para.B * 2;
             long long gwarps = std::min<long long>(148LL * 16, std::max<long long>(1, (1LL << 28) / (slot_floats * 4)));

@@ -9,6 +9,7 @@
 #include "vbm.cuh"
 #include "cf.cuh"
 #include "cf_box.cuh"
+#include "cf_mid.cuh"
 #include "cf_tc.cuh"
 #include "fp64.cuh"
 #include "convert.cuh"
@@ -19,6 +20,7 @@
 #include <atomic>
 #include <cmath>
 #include <cstring>
+#include <type_traits>
 #include <vector>
 
 namespace bm3d {
@@ -437,6 +439,33 @@ cudaError_t launch_cf_fp64(const CFArgs &a, const F64Args &f, cudaStream_t s)
     COUNT_LAUNCH();
     finalize_fp64_kernel<<<grid, 128, 0, s>>>(f, a.W, a.H, 1, a.process[0], a.process[1], a.process[2]);
     return cudaGetLastError();
+}
+
+template <int BM, bool DIRECT>
+static cudaError_t launch_cf_mid_t(const CFArgs &a, cudaStream_t s)
+{
+    auto kernel = a.wiener ? cf_mid_kernel<BM, DIRECT, true> : cf_mid_kernel<BM, DIRECT, false>;
+    const size_t smem = mid_smem_bytes(BM, a.B, a.G, a.wiener);
+    cudaError_t e;
+    if ((e = allow_smem(kernel, smem)) != cudaSuccess) return e;
+    COUNT_LAUNCH();
+    kernel<<<(unsigned)std::max<long long>(1, std::min<long long>(a.ngroups, 148LL * 64)), kMidThreads, smem, s>>>(a);
+    return cudaGetLastError();
+}
+
+int launch_cf_mid(const CFArgs &a, cudaStream_t s, cudaError_t *e)
+{
+    if (a.B < 2 || a.B > 16 || a.G > 32 || mid_smem_bytes(16, a.B, a.G, a.wiener) > 200 * 1024) return 0;
+    switch (a.B) {
+    case 2: *e = launch_cf_mid_t<2, false>(a, s); break;
+    case 4: *e = launch_cf_mid_t<4, false>(a, s); break;
+    case 8: *e = launch_cf_mid_t<8, false>(a, s); break;
+    case 16: *e = launch_cf_mid_t<16, false>(a, s); break;
+    default:
+        *e = a.B < 4 ? launch_cf_mid_t<4, true>(a, s) : a.B < 8 ? launch_cf_mid_t<8, true>(a, s)
+           : a.B <= 12 ? launch_cf_mid_t<12, true>(a, s) : launch_cf_mid_t<16, true>(a, s);
+    }
+    return 1;
 }
 
 cudaError_t launch_cf_generic(const CFArgs &a, int warps, int grid, cudaStream_t s)

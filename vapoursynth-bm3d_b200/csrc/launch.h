@@ -41,6 +41,9 @@ int launch_cf_box(const CFArgs &a, const CFBox &g, int step, cudaStream_t s, cud
 cudaError_t launch_cf_fast(const CFArgs &a, cudaStream_t s);
 // Indices of the groups with count < G into list (device counter n, zeroed by the caller).
 cudaError_t launch_cf_partial_list(const int *count, long long ngroups, int G, long long *list, unsigned int *n, cudaStream_t s);
+// Groups of at most 32 blocks of 2 x 2 to 16 x 16 in shared memory, a CTA per group; returns 0 if the shape is
+// not its own, else 1 and the status.
+int launch_cf_mid(const CFArgs &a, cudaStream_t s, cudaError_t *e);
 cudaError_t launch_cf_generic(const CFArgs &a, int warps, int grid, cudaStream_t s);
 cudaError_t launch_convert(const ConvProgram &pr, const PlanePtr *in_dev, const PlanePtr *out_dev,
                            int nframes, cudaStream_t s);
