@@ -231,6 +231,12 @@ struct ConvProgram {
     int W, H;
 };
 
+// Planes of one conversion launch, frame by frame: up to kConvPlanes per side (8 frames of three planes)
+constexpr int kConvPlanes = 24;
+struct ConvTable {
+    PlanePtr in[kConvPlanes], out[kConvPlanes];
+};
+
 // finalize: out = num / box_B(wmap) for processed planes of a batch of frames.
 // FP64 oracle outputs and constants (inspection only)
 struct F64Args {

@@ -15,22 +15,6 @@ namespace bm3d {
 
 
 
-__device__ __forceinline__ float load_sample(const PlanePtr &p, int kind, int y, int x)
-{
-    const char *row = static_cast<const char *>(p.ptr) + (long long)y * p.stride;
-    if (kind == SK_U8) return (float)reinterpret_cast<const uint8_t *>(row)[x];
-    if (kind == SK_U16) return (float)reinterpret_cast<const uint16_t *>(row)[x];
-    return reinterpret_cast<const float *>(row)[x];
-}
-
-__device__ __forceinline__ void store_sample(const PlanePtr &p, int kind, int y, int x, float v)
-{
-    char *row = static_cast<char *>(p.ptr) + (long long)y * p.stride;
-    if (kind == SK_U8) reinterpret_cast<uint8_t *>(row)[x] = (uint8_t)v;       // truncation, as static_cast
-    else if (kind == SK_U16) reinterpret_cast<uint16_t *>(row)[x] = (uint16_t)v;
-    else reinterpret_cast<float *>(row)[x] = v;
-}
-
 __device__ __forceinline__ float clip_ref(float v, float lo, float hi)
 {
     // Clip() of include/Helper.h:395-399
@@ -39,65 +23,142 @@ __device__ __forceinline__ float clip_ref(float v, float lo, float hi)
 
 
 
-__global__ void convert_kernel(ConvProgram pr, const PlanePtr *in, const PlanePtr *out)
+// Eight samples of a row.  VEC: consecutive ones, read and written with 16-byte accesses where the eight fit
+// in the row (8 bytes for 8-bit samples; the host checks the alignment of every plane); else
+// samples t, t + rw, t + 2 rw ... of the row's rw threads, so that a warp's accesses stay contiguous.
+struct RowSpan {
+    int t, rw, W;
+    template <bool VEC> __device__ __forceinline__ int at(int k) const { return VEC ? 8 * t + k : t + k * rw; }
+};
+
+template <bool VEC>
+__device__ __forceinline__ void load8(const PlanePtr &p, int kind, int y, const RowSpan &r, float (&v)[8])
 {
-    const int f = blockIdx.z;
-    const int y = blockIdx.y;
-    const PlanePtr *pi = in + f * pr.nin;
-    const PlanePtr *po = out + f * pr.nout;
-    for (int x = blockIdx.x * blockDim.x + threadIdx.x; x < pr.W; x += gridDim.x * blockDim.x) {
-        if (pr.raw) {
-            for (int c = 0; c < pr.nin; ++c) {
-                if (!po[c].ptr) continue;
-                const char *si = static_cast<const char *>(pi[c].ptr) + (long long)y * pi[c].stride;
-                char *so = static_cast<char *>(po[c].ptr) + (long long)y * po[c].stride;
-                if (pr.in_kind == SK_U8) reinterpret_cast<uint8_t *>(so)[x] = reinterpret_cast<const uint8_t *>(si)[x];
-                else if (pr.in_kind == SK_U16) reinterpret_cast<uint16_t *>(so)[x] = reinterpret_cast<const uint16_t *>(si)[x];
-                else reinterpret_cast<float *>(so)[x] = reinterpret_cast<const float *>(si)[x];
-            }
-        } else if (pr.mode == 0) {
-            for (int c = 0; c < pr.nin; ++c) {
-                if (!po[c].ptr) continue;
-                const LinearOp &o = pr.op[c];
-                float t = __fadd_rn(__fmul_rn(load_sample(pi[c], pr.in_kind, y, x), o.gain), o.offset);
-                if (o.clip) t = clip_ref(t, o.lo, o.hi);
-                store_sample(po[c], pr.out_kind, y, x, t);
-            }
-        } else if (pr.mode == 1 || pr.mode == 2) {
-            const float R = load_sample(pi[0], pr.in_kind, y, x);
-            const float Gc = load_sample(pi[1], pr.in_kind, y, x);
-            const float Bc = load_sample(pi[2], pr.in_kind, y, x);
-            float t = __fadd_rn(__fmul_rn(__fadd_rn(__fadd_rn(R, Gc), Bc), pr.op[0].gain), pr.op[0].offset);
-            if (pr.op[0].clip) t = clip_ref(t, pr.op[0].lo, pr.op[0].hi);
-            store_sample(po[0], pr.out_kind, y, x, t);
-            if (pr.mode == 1) {
-                float u = __fadd_rn(__fmul_rn(__fsub_rn(R, Bc), pr.op[1].gain), pr.op[1].offset);
-                if (pr.op[1].clip) u = clip_ref(u, pr.op[1].lo, pr.op[1].hi);
-                if (po[1].ptr) store_sample(po[1], pr.out_kind, y, x, u);
-                float v = __fadd_rn(__fmul_rn(__fadd_rn(__fsub_rn(R, __fmul_rn(Gc, 2.0f)), Bc), pr.op[2].gain), pr.op[2].offset);
-                if (pr.op[2].clip) v = clip_ref(v, pr.op[2].lo, pr.op[2].hi);
-                if (po[2].ptr) store_sample(po[2], pr.out_kind, y, x, v);
-            }
+    const char *row = static_cast<const char *>(p.ptr) + (long long)y * p.stride;
+    if (VEC && 8 * r.t + 8 <= r.W) {
+        if (kind == SK_U8) {
+            const uint2 q = reinterpret_cast<const uint2 *>(row)[r.t];
+#pragma unroll
+            for (int k = 0; k < 8; ++k) v[k] = (float)(((k < 4 ? q.x : q.y) >> (8 * (k & 3))) & 0xffu);
+        } else if (kind == SK_U16) {
+            const uint4 q = reinterpret_cast<const uint4 *>(row)[r.t];
+            const uint32_t w[4] = {q.x, q.y, q.z, q.w};
+#pragma unroll
+            for (int k = 0; k < 8; ++k) v[k] = (float)((w[k >> 1] >> (16 * (k & 1))) & 0xffffu);
         } else {
-            const float Y = load_sample(pi[0], pr.in_kind, y, x);
-            const float U = load_sample(pi[1], pr.in_kind, y, x);
-            const float V = load_sample(pi[2], pr.in_kind, y, x);
-            const float *k = pr.coef;
-            float r = __fadd_rn(__fadd_rn(__fadd_rn(__fmul_rn(k[0], Y), __fmul_rn(k[1], U)), __fmul_rn(k[2], V)), pr.off[0]);
-            float g = __fadd_rn(__fadd_rn(__fmul_rn(k[3], Y), __fmul_rn(k[5], V)), pr.off[1]);
-            float b = __fadd_rn(__fadd_rn(__fadd_rn(__fmul_rn(k[6], Y), __fmul_rn(k[7], U)), __fmul_rn(k[8], V)), pr.off[2]);
-            if (pr.op[0].clip) {
-                r = clip_ref(r, pr.op[0].lo, pr.op[0].hi);
-                g = clip_ref(g, pr.op[0].lo, pr.op[0].hi);
-                b = clip_ref(b, pr.op[0].lo, pr.op[0].hi);
-            }
-            store_sample(po[0], pr.out_kind, y, x, r);
-            store_sample(po[1], pr.out_kind, y, x, g);
-            store_sample(po[2], pr.out_kind, y, x, b);
+            const float4 a = reinterpret_cast<const float4 *>(row)[2 * r.t], b = reinterpret_cast<const float4 *>(row)[2 * r.t + 1];
+            v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
+            v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
         }
+        return;
+    }
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+        const int x = r.at<VEC>(k);
+        if (x >= r.W) continue;
+        v[k] = kind == SK_U8 ? (float)reinterpret_cast<const uint8_t *>(row)[x]
+             : kind == SK_U16 ? (float)reinterpret_cast<const uint16_t *>(row)[x] : reinterpret_cast<const float *>(row)[x];
     }
 }
 
+// integer samples by truncation, as static_cast
+template <bool VEC>
+__device__ __forceinline__ void store8(const PlanePtr &p, int kind, int y, const RowSpan &r, const float (&v)[8])
+{
+    char *row = static_cast<char *>(p.ptr) + (long long)y * p.stride;
+    if (VEC && 8 * r.t + 8 <= r.W) {
+        if (kind == SK_U8) {
+            uint32_t w[2] = {0u, 0u};
+#pragma unroll
+            for (int k = 0; k < 8; ++k) w[k >> 2] |= (uint32_t)(uint8_t)v[k] << (8 * (k & 3));
+            reinterpret_cast<uint2 *>(row)[r.t] = make_uint2(w[0], w[1]);
+        } else if (kind == SK_U16) {
+            uint32_t w[4] = {0u, 0u, 0u, 0u};
+#pragma unroll
+            for (int k = 0; k < 8; ++k) w[k >> 1] |= (uint32_t)(uint16_t)v[k] << (16 * (k & 1));
+            reinterpret_cast<uint4 *>(row)[r.t] = make_uint4(w[0], w[1], w[2], w[3]);
+        } else {
+            reinterpret_cast<float4 *>(row)[2 * r.t] = make_float4(v[0], v[1], v[2], v[3]);
+            reinterpret_cast<float4 *>(row)[2 * r.t + 1] = make_float4(v[4], v[5], v[6], v[7]);
+        }
+        return;
+    }
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+        const int x = r.at<VEC>(k);
+        if (x >= r.W) continue;
+        if (kind == SK_U8) reinterpret_cast<uint8_t *>(row)[x] = (uint8_t)v[k];
+        else if (kind == SK_U16) reinterpret_cast<uint16_t *>(row)[x] = (uint16_t)v[k];
+        else reinterpret_cast<float *>(row)[x] = v[k];
+    }
+}
+
+__device__ __forceinline__ float linear_ref(float t, const LinearOp &o)
+{
+    t = __fadd_rn(__fmul_rn(t, o.gain), o.offset);
+    return o.clip ? clip_ref(t, o.lo, o.hi) : t;
+}
+
+// One thread per eight samples of a row, one grid row per frame; the planes' addresses come with the launch.
+// Bound: HBM.  4 frames of 1920x1080 RGB, 16 bits -> float OPP -> 16 bits, 300 MB with the intermediate: a pixel per
+// thread and address tables copied to the device first 97 us, 54 us now.
+template <bool VEC>
+__global__ void __launch_bounds__(256) convert_kernel(const __grid_constant__ ConvProgram pr, const __grid_constant__ ConvTable tab)
+{
+    const int rw = (pr.W + 7) >> 3, u = blockIdx.x * blockDim.x + threadIdx.x;
+    const int y = u / rw, f = blockIdx.y;
+    if (y >= pr.H) return;
+    const RowSpan r{u - y * rw, rw, pr.W};
+    const int i0 = f * pr.nin, o0 = f * pr.nout;
+    if (pr.raw || pr.mode == 0) {
+        for (int c = 0; c < pr.nin; ++c) {
+            if (!tab.out[o0 + c].ptr) continue;
+            float v[8];
+            load8<VEC>(tab.in[i0 + c], pr.in_kind, y, r, v);
+            if (!pr.raw) {
+#pragma unroll
+                for (int k = 0; k < 8; ++k) v[k] = linear_ref(v[k], pr.op[c]);
+            }
+            store8<VEC>(tab.out[o0 + c], pr.out_kind, y, r, v);
+        }
+        return;
+    }
+    float a[8], b[8], c[8];
+    load8<VEC>(tab.in[i0], pr.in_kind, y, r, a);
+    load8<VEC>(tab.in[i0 + 1], pr.in_kind, y, r, b);
+    load8<VEC>(tab.in[i0 + 2], pr.in_kind, y, r, c);
+    if (pr.mode == 1 || pr.mode == 2) {
+        float Y[8], U[8], V[8];
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+            Y[k] = linear_ref(__fadd_rn(__fadd_rn(a[k], b[k]), c[k]), pr.op[0]);
+            U[k] = linear_ref(__fsub_rn(a[k], c[k]), pr.op[1]);
+            V[k] = linear_ref(__fadd_rn(__fsub_rn(a[k], __fmul_rn(b[k], 2.0f)), c[k]), pr.op[2]);
+        }
+        store8<VEC>(tab.out[o0], pr.out_kind, y, r, Y);
+        if (pr.mode == 1) {
+            if (tab.out[o0 + 1].ptr) store8<VEC>(tab.out[o0 + 1], pr.out_kind, y, r, U);
+            if (tab.out[o0 + 2].ptr) store8<VEC>(tab.out[o0 + 2], pr.out_kind, y, r, V);
+        }
+        return;
+    }
+    const float *m = pr.coef;
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+        const float Y = a[k], U = b[k], V = c[k];
+        a[k] = __fadd_rn(__fadd_rn(__fadd_rn(__fmul_rn(m[0], Y), __fmul_rn(m[1], U)), __fmul_rn(m[2], V)), pr.off[0]);
+        b[k] = __fadd_rn(__fadd_rn(__fmul_rn(m[3], Y), __fmul_rn(m[5], V)), pr.off[1]);
+        c[k] = __fadd_rn(__fadd_rn(__fadd_rn(__fmul_rn(m[6], Y), __fmul_rn(m[7], U)), __fmul_rn(m[8], V)), pr.off[2]);
+        if (pr.op[0].clip) {
+            a[k] = clip_ref(a[k], pr.op[0].lo, pr.op[0].hi);
+            b[k] = clip_ref(b[k], pr.op[0].lo, pr.op[0].hi);
+            c[k] = clip_ref(c[k], pr.op[0].lo, pr.op[0].hi);
+        }
+    }
+    store8<VEC>(tab.out[o0], pr.out_kind, y, r, a);
+    store8<VEC>(tab.out[o0 + 1], pr.out_kind, y, r, b);
+    store8<VEC>(tab.out[o0 + 2], pr.out_kind, y, r, c);
+}
 
 // Tile of the denominator (the B x B box sum of the per-origin weight map wm) for output rows
 // [ty0, ty0 + kFinTH) and columns [tx0, tx0 + kFinTW): the weight region with its (B - 1) halo is

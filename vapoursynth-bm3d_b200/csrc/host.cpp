@@ -602,6 +602,23 @@ public:
     }
 
 protected:
+    // float planes (np per frame) to the output format of VAggregate, float or 16 bits by every frame's
+    // range flag; frames of equal flags in one conversion
+    void float_egress(const std::vector<PlanePtr> &in, const std::vector<PlanePtr> &out, const std::vector<bool> &full, int np,
+                      int sample, int W, int H)
+    {
+        const int count = (int)full.size();
+        for (int k = 0, e; k < count; k = e) {
+            for (e = k + 1; e < count && (sample == 1 || full[e] == full[k]); ++e) {}
+            ConvProgram pr = raw_program(SK_F32, np, W, H);
+            if (sample != 1) {
+                pr.raw = 0;
+                pr.out_kind = SK_U16;
+                for (int p = 0; p < np; ++p) pr.op[p] = float2int_op(16, full[k], p > 0);
+            }
+            CU(launch_convert(pr, in.data() + k * np, out.data() + k * np, e - k, stream));
+        }
+    }
     Stager stager_;
     DevBuf ptr_in_, ptr_out_;
     // uploads a PlanePtr table to the device (small)
@@ -686,7 +703,7 @@ public:
         const ConvProgram pr = to_opp
             ? rgb2opp_program(sample_kind(vi), vi.bits_per_sample, sample_kind(ovi), ovi.bits_per_sample, W, H, false)
             : opp2rgb_program(sample_kind(vi), vi.bits_per_sample, sample_kind(ovi), ovi.bits_per_sample, W, H);
-        CU(launch_convert(pr, upload_ptrs(ptr_in_, in), upload_ptrs(ptr_out_, out), count, stream));
+        CU(launch_convert(pr, in.data(), out.data(), count, stream));
         stager_.flush(stream);
         for (int k = 0; k < count; ++k) {
             copy_props(src[k], dst[k]);
@@ -927,7 +944,15 @@ public:
     // ---- workspace ----
     int W = 0, H = 0, ld = 0;
     long long fs = 0;                      // floats per frame plane
-    DevBuf ws_src[3], ws_ref[3], acc_num[3], acc_w[3];
+    DevBuf ws_src[3], ws_ref[3];
+    // accumulators: numerator and weight map of every processed plane, one after the other, cleared by one memset
+    struct AccView {
+        float *p = nullptr;
+        template <typename T> T *as() const { return p; }
+    };
+    AccView acc_num[3], acc_w[3];
+    DevBuf acc_buf;
+    size_t acc_bytes = 0;
     DevBuf m_pos, m_n, m_key, v_pos, v_n, v_key;
     DevBuf d_sy, d_sx, scratch;
     DevBuf d_winb, d_winl, d_winc, d_slot0;
@@ -1026,8 +1051,7 @@ public:
                 out.push_back(PlanePtr{ws[p].as<float>() + slot * fs, (long long)ld * 4});
             const ConvProgram pr = y_only ? rgb2y_program(kind, vi.bits_per_sample, W, H)
                                           : rgb2opp_program(kind, vi.bits_per_sample, SK_F32, 32, W, H, false);
-            CU(launch_convert(pr, upload_ptrs(conv_in_[conv_i_], in), upload_ptrs(conv_out_[conv_i_], out), 1, stream));
-            conv_i_ = (conv_i_ + 1) % kConvSlots;
+            CU(launch_convert(pr, in.data(), out.data(), 1, stream));
             return;
         }
         for (int p = 0; p < np; ++p) {
@@ -1050,8 +1074,7 @@ public:
                 pr.H = H;
                 pr.op[0] = int2float_op(vi.bits_per_sample, full, p > 0);
             }
-            CU(launch_convert(pr, upload_ptrs(conv_in_[conv_i_], i1), upload_ptrs(conv_out_[conv_i_], o1), 1, stream));
-            conv_i_ = (conv_i_ + 1) % kConvSlots;
+            CU(launch_convert(pr, i1.data(), o1.data(), 1, stream));
         }
     }
 
@@ -1099,8 +1122,7 @@ public:
                     out.push_back(need ? PlanePtr{ws[p].as<float>() + (slot0 + k) * fs, (long long)ld * 4} : PlanePtr{nullptr, 0});
                 }
         }
-        CU(launch_convert(pr, upload_ptrs(conv_in_[conv_i_], in), upload_ptrs(conv_out_[conv_i_], out), count, stream));
-        conv_i_ = (conv_i_ + 1) % kConvSlots;
+        CU(launch_convert(pr, in.data(), out.data(), count, stream));
     }
 
     // BM3D_Process_Base::NewFrame / VBM3D_Process_Base::NewFrame property handling
@@ -1126,6 +1148,22 @@ public:
         m_n.get(sizeof(int) * nb);
         m_key.get(sizeof(float) * nb * para.G);
     }
+
+    // room for `planes` accumulator planes of every processed colour plane
+    void ensure_acc(long long planes)
+    {
+        int np = 0;
+        for (int p = 0; p < nplanes(); ++p) np += process[p] != 0;
+        acc_bytes = sizeof(float) * (size_t)fs * planes * 2 * np;
+        float *at = static_cast<float *>(acc_buf.get(acc_bytes));
+        for (int p = 0; p < nplanes(); ++p)
+            if (process[p]) {
+                acc_num[p].p = at;
+                acc_w[p].p = at + fs * planes;
+                at += 2 * fs * planes;
+            }
+    }
+    void clear_acc() { CU(cudaMemsetAsync(acc_buf.p, 0, acc_bytes, stream)); }
 
     bool learned_matching() const { return learned && para.B == 8 && para.G >= 2 && para.G <= 32; }
 
@@ -1242,12 +1280,27 @@ public:
         a.dtab = dtabs.tab.as<float>();
         a.dtab_off = dtabs.off.as<int>();
         const bool fast = cf_fast_supported(para.B, para.G);
-        if (!wiener) {
-            // retained counts of every group (inspection), written by the filter kernels
-            a.retained = static_cast<int *>(retained_buf.get(sizeof(int) * 3 * (size_t)std::max<long long>(1, ngroups)));
-            CU(cudaMemsetAsync(a.retained, 0xff, sizeof(int) * 3 * (size_t)std::max<long long>(1, ngroups), stream));
+        // retained counts of every group (inspection), written by the filter kernels
+        if (!wiener) a.retained = static_cast<int *>(retained_buf.get(sizeof(int) * 3 * (size_t)std::max<long long>(1, ngroups)));
+        const bool tensor = fast && tc && tc_tab.p;
+        if (fast && !v && !tensor) {
+            CFBox g{};
+            g.scan_y = d_sy.as<int>();
+            g.scan_x = d_sx.as<int>();
+            g.nby = (int)sy.size();
+            g.nbx = (int)sx.size();
+            g.range = para.R / para.bmstep * para.bmstep;
+            for (int p = 0; p < 3; ++p)
+                if (a.process[p]) g.plane[g.nplanes++] = p;
+            cudaError_t e = cudaSuccess;
+            if (launch_cf_box(a, g, para.step, stream, &e)) {
+                CU(e);
+                return;
+            }
         }
-        if (fast && tc && tc_tab.p) {
+        // kernels that leave counts out (the box form writes every processed plane's)
+        if (!wiener) CU(cudaMemsetAsync(a.retained, 0xff, sizeof(int) * 3 * (size_t)std::max<long long>(1, ngroups), stream));
+        if (tensor) {
             a.recheck_band = recheck_band;
             a.tc_stats = static_cast<unsigned long long *>(tc_counts.get(2 * sizeof(unsigned long long)));
             CU(cudaMemsetAsync(a.tc_stats, 0, 2 * sizeof(unsigned long long), stream));
@@ -1279,21 +1332,6 @@ public:
             CU(launch_cf_partial_list(cnt, ngroups, para.G, pl, pn, stream));
             a.plist = pl;
             a.plist_n = pn;
-        }
-        if (fast && !v && !a.plist) {
-            CFBox g{};
-            g.scan_y = d_sy.as<int>();
-            g.scan_x = d_sx.as<int>();
-            g.nby = (int)sy.size();
-            g.nbx = (int)sx.size();
-            g.range = para.R / para.bmstep * para.bmstep;
-            for (int p = 0; p < 3; ++p)
-                if (a.process[p]) g.plane[g.nplanes++] = p;
-            cudaError_t e = cudaSuccess;
-            if (launch_cf_box(a, g, para.step, stream, &e)) {
-                CU(e);
-                return;
-            }
         }
         if (fast) CU(launch_cf_fast(a, stream));
         cudaError_t mid = cudaSuccess;
@@ -1365,7 +1403,9 @@ public:
         CU(cudaStreamSynchronize(stream));
         const size_t ng = nb * last_count;
         for (int p = 0; p < 3; ++p)
-            CU(cudaMemcpy(out + p * nb, retained_buf.as<int>() + p * ng + k * nb, sizeof(int) * nb, cudaMemcpyDeviceToHost));
+            if (process[p] && p < nplanes())
+                CU(cudaMemcpy(out + p * nb, retained_buf.as<int>() + p * ng + k * nb, sizeof(int) * nb, cudaMemcpyDeviceToHost));
+            else std::fill(out + p * nb, out + (p + 1) * nb, -1);
         return (int)nb;
     }
 
@@ -1402,9 +1442,6 @@ public:
     }
 
 protected:
-    static constexpr int kConvSlots = 64;
-    DevBuf conv_in_[kConvSlots], conv_out_[kConvSlots];
-    int conv_i_ = 0;
 };
 
 // ---------------------------------------------------------------------------------------------
@@ -1439,8 +1476,7 @@ public:
             for (int k = 0; k < count; ++k) {
                 std::vector<PlanePtr> i1, o1;
                 for (int p = 0; p < np; ++p) { i1.push_back(stager_.view(*src[k], p, g, stream)); o1.push_back(stager_.target(*dst[k], p, g)); }
-                CU(launch_convert(raw_program(sample_kind(vi), np, W, H), upload_ptrs(conv_in_[conv_i_], i1), upload_ptrs(conv_out_[conv_i_], o1), 1, stream));
-                conv_i_ = (conv_i_ + 1) % kConvSlots;
+                CU(launch_convert(raw_program(sample_kind(vi), np, W, H), i1.data(), o1.data(), 1, stream));
                 copy_props(src[k], dst[k]);
             }
             stager_.flush(stream);
@@ -1448,11 +1484,7 @@ public:
             return BM3D_OK;
         }
         ensure_ws(count, count);
-        for (int p = 0; p < 3; ++p)
-            if (process[p] && p < np) {
-                acc_num[p].get(sizeof(float) * fs * count);
-                acc_w[p].get(sizeof(float) * fs * count);
-            }
+        ensure_acc(count);
         CU(cudaMemsetAsync(stats, 0, 3 * sizeof(unsigned long long), stream));
         mark(0);
         std::vector<bool> full(count);
@@ -1463,11 +1495,7 @@ public:
         run_bm(0, count, m_pos.as<uint32_t>(), m_n.as<int>(), m_key.as<float>());
         mark(2);
         mark(3);
-        for (int p = 0; p < np; ++p)
-            if (process[p]) {
-                CU(cudaMemsetAsync(acc_num[p].p, 0, sizeof(float) * fs * count, stream));
-                CU(cudaMemsetAsync(acc_w[p].p, 0, sizeof(float) * fs * count, stream));
-            }
+        clear_acc();
         const long long bpf = (long long)sy.size() * sx.size();
         run_cf(bpf * count, bpf, m_pos.as<uint32_t>(), m_n.as<int>(), false, nullptr, nullptr, 1, 0);
         mark(4);
@@ -1505,8 +1533,7 @@ public:
                 pr.mode = 0; pr.in_kind = SK_F32; pr.out_kind = kind; pr.nin = pr.nout = np; pr.W = W; pr.H = H;
                 for (int p = 0; p < np; ++p) pr.op[p] = float2int_op(vi.bits_per_sample, full[0], p > 0);
             }
-            CU(launch_convert(pr, upload_ptrs(conv_in_[conv_i_], i1), upload_ptrs(conv_out_[conv_i_], o1), count, stream));
-            conv_i_ = (conv_i_ + 1) % kConvSlots;
+            CU(launch_convert(pr, i1.data(), o1.data(), count, stream));
         }
         for (int k = 0; k < count; ++k) {
             if (batch) {
@@ -1518,8 +1545,7 @@ public:
                 for (int p = 0; p < 3; ++p) i1.push_back(PlanePtr{acc_num[p].as<float>() + k * fs, (long long)ld * 4});
                 for (int p = 0; p < 3; ++p) o1.push_back(stager_.target(*dst[k], p, g));
                 CU(launch_convert(opp2rgb_program(SK_F32, 32, kind, vi.bits_per_sample, W, H),
-                                  upload_ptrs(conv_in_[conv_i_], i1), upload_ptrs(conv_out_[conv_i_], o1), 1, stream));
-                conv_i_ = (conv_i_ + 1) % kConvSlots;
+                                  i1.data(), o1.data(), 1, stream));
             } else {
                 for (int p = 0; p < np; ++p) {
                     std::vector<PlanePtr> a1, b1;
@@ -1537,8 +1563,7 @@ public:
                         a1.push_back(stager_.view(*src[k], p, g, stream));
                         pr = raw_program(kind, 1, W, H);
                     }
-                    CU(launch_convert(pr, upload_ptrs(conv_in_[conv_i_], a1), upload_ptrs(conv_out_[conv_i_], b1), 1, stream));
-                    conv_i_ = (conv_i_ + 1) % kConvSlots;
+                    CU(launch_convert(pr, a1.data(), b1.data(), 1, stream));
                 }
             }
             copy_props(src[k], dst[k]);
@@ -1631,11 +1656,7 @@ public:
         v_pos.get(sizeof(uint32_t) * nb * para.G);
         v_n.get(sizeof(int) * nb);
         v_key.get(sizeof(float) * nb * para.G);
-        for (int p = 0; p < 3; ++p)
-            if (process[p] && p < np) {
-                acc_num[p].get(sizeof(float) * fs * acc_planes);
-                acc_w[p].get(sizeof(float) * fs * acc_planes);
-            }
+        ensure_acc(acc_planes);
         CU(cudaMemsetAsync(stats, 0, 3 * sizeof(unsigned long long), stream));
         // window frames into the workspace; properties of each output frame's own source frame
         std::vector<bool> full(nwin);
@@ -1727,11 +1748,7 @@ public:
         CU(launch_vbm_predict(va, fast_ps, rc, smem, stream));
         mark(3);
         // K3+K4 into the accumulators
-        for (int p = 0; p < np; ++p)
-            if (process[p]) {
-                CU(cudaMemsetAsync(acc_num[p].p, 0, sizeof(float) * fs * acc_planes, stream));
-                CU(cudaMemsetAsync(acc_w[p].p, 0, sizeof(float) * fs * acc_planes, stream));
-            }
+        clear_acc();
         const long long bpf = (long long)sy.size() * sx.size();
         run_cf(bpf * rc, bpf, v_pos.as<uint32_t>(), v_n.as<int>(), true, d_winb.as<int>(), d_slot0.as<int>(),
                aggregate ? 0 : slots, fs);
@@ -1823,27 +1840,20 @@ private:
         fa.B = para.B;
         CU(launch_finalize(fa, count, stream));
         const PlaneGeom go{W * bytes_per_sample(ovi), H};
+        std::vector<PlanePtr> in, out;
+        std::vector<bool> full(count);
         for (int k = 0; k < count; ++k) {
             const bm3d_frame &sf = *src[n + k - first];
             const int64_t opp = vi.color_family == BM3D_RGB ? 1 : (sf.prop_bm3d_opp < 0 ? 0 : sf.prop_bm3d_opp);
-            const bool full = (sf.prop_range < 0 || opp == 1) ? true : sf.prop_range != 0;
+            full[k] = (sf.prop_range < 0 || opp == 1) ? true : sf.prop_range != 0;
             for (int p = 0; p < np; ++p) {
                 PlanePtr t = stager_.target(*dst[k], p, go);
-                if (!process[p]) {
-                    CU(cudaMemset2DAsync(t.ptr, t.stride, 0, (size_t)go.width_bytes, H, stream));
-                    continue;
-                }
-                std::vector<PlanePtr> a1{PlanePtr{agg[p] + (long long)k * fs, (long long)ld * 4}}, b1{t};
-                ConvProgram pr{};
-                if (agg_sample == 1) pr = raw_program(SK_F32, 1, W, H);
-                else {
-                    pr.mode = 0; pr.in_kind = SK_F32; pr.out_kind = SK_U16; pr.nin = pr.nout = 1; pr.W = W; pr.H = H;
-                    pr.op[0] = float2int_op(16, full, p > 0);
-                }
-                CU(launch_convert(pr, upload_ptrs(conv_in_[conv_i_], a1), upload_ptrs(conv_out_[conv_i_], b1), 1, stream));
-                conv_i_ = (conv_i_ + 1) % kConvSlots;
+                if (!process[p]) CU(cudaMemset2DAsync(t.ptr, t.stride, 0, (size_t)go.width_bytes, H, stream));
+                in.push_back(PlanePtr{process[p] ? agg[p] + (long long)k * fs : nullptr, (long long)ld * 4});
+                out.push_back(process[p] ? t : PlanePtr{nullptr, 0});
             }
         }
+        float_egress(in, out, full, np, agg_sample, W, H);
     }
 
     bool frame_full_quiet(const bm3d_frame &fr) const
@@ -1963,36 +1973,26 @@ public:
         a.W = W;
         a.radius = radius;
         CU(launch_vaggregate(a, count, stream));
+        std::vector<PlanePtr> ci, co;
         for (int k = 0; k < count; ++k) {
             for (int p = 0; p < np; ++p) {
                 PlanePtr t = stager_.target(*dst[k], p, go);
-                if (!proc[p]) {
-                    CU(cudaMemset2DAsync(t.ptr, t.stride, 0, (size_t)go.width_bytes, Ho, stream));
-                    continue;
-                }
-                std::vector<PlanePtr> a1{PlanePtr{ws[p].as<float>() + k * fs, (long long)ld * 4}}, b1{t};
-                ConvProgram pr{};
-                if (sample == 1) pr = raw_program(SK_F32, 1, W, Ho);
-                else {
-                    pr.mode = 0; pr.in_kind = SK_F32; pr.out_kind = SK_U16; pr.nin = pr.nout = 1; pr.W = W; pr.H = Ho;
-                    pr.op[0] = float2int_op(16, full[k], p > 0);
-                }
-                CU(launch_convert(pr, upload_ptrs(conv_in_[conv_i_], a1), upload_ptrs(conv_out_[conv_i_], b1), 1, stream));
-                conv_i_ = (conv_i_ + 1) % kConvSlots;
+                if (!proc[p]) CU(cudaMemset2DAsync(t.ptr, t.stride, 0, (size_t)go.width_bytes, Ho, stream));
+                ci.push_back(PlanePtr{proc[p] ? ws[p].as<float>() + k * fs : nullptr, (long long)ld * 4});
+                co.push_back(proc[p] ? t : PlanePtr{nullptr, 0});
             }
             copy_props(src[n + k - first], dst[k]);
             dst[k]->prop_v_radius = -1;
             dst[k]->prop_v_process_count = -1;
         }
+        float_egress(ci, co, full, np, sample, W, Ho);
         stager_.flush(stream);
         if (sync) { CU(cudaStreamSynchronize(stream)); stager_.release(); }
         return BM3D_OK;
     }
 
 private:
-    static constexpr int kConvSlots = 64;
-    DevBuf conv_in_[kConvSlots], conv_out_[kConvSlots], hdrbuf_;
-    int conv_i_ = 0;
+    DevBuf hdrbuf_;
 };
 
 }  // namespace bm3d

@@ -475,13 +475,31 @@ cudaError_t launch_cf_generic(const CFArgs &a, int warps, int grid, cudaStream_t
     return cudaGetLastError();
 }
 
-cudaError_t launch_convert(const ConvProgram &pr, const PlanePtr *in, const PlanePtr *out, int nframes,
-                           cudaStream_t s)
+cudaError_t launch_convert(const ConvProgram &pr, const PlanePtr *in, const PlanePtr *out, int nframes, cudaStream_t s)
 {
-    dim3 block(256);
-    dim3 grid((pr.W + 255) / 256, pr.H, nframes);
-    COUNT_LAUNCH();
-    convert_kernel<<<grid, block, 0, s>>>(pr, in, out);
+    auto aligned = [](const PlanePtr &p, int kind) {
+        const long long m = kind == SK_U8 ? 7 : 15;
+        return !p.ptr || ((reinterpret_cast<long long>(p.ptr) | p.stride) & m) == 0;
+    };
+    const int per = kConvPlanes / std::max(pr.nin, pr.nout);
+    const long long units = (long long)((pr.W + 7) >> 3) * pr.H;
+    for (int f0 = 0; f0 < nframes; f0 += per) {
+        const int nf = std::min(per, nframes - f0);
+        ConvTable t{};
+        bool vec = true;
+        for (int k = 0; k < nf * pr.nin; ++k) {
+            t.in[k] = in[f0 * pr.nin + k];
+            vec = vec && aligned(t.in[k], pr.in_kind);
+        }
+        for (int k = 0; k < nf * pr.nout; ++k) {
+            t.out[k] = out[f0 * pr.nout + k];
+            vec = vec && aligned(t.out[k], pr.out_kind);
+        }
+        const dim3 grid((unsigned)((units + 255) / 256), nf);
+        COUNT_LAUNCH();
+        if (vec) convert_kernel<true><<<grid, 256, 0, s>>>(pr, t);
+        else convert_kernel<false><<<grid, 256, 0, s>>>(pr, t);
+    }
     return cudaGetLastError();
 }
 

@@ -45,8 +45,8 @@ cudaError_t launch_cf_partial_list(const int *count, long long ngroups, int G, l
 // not its own, else 1 and the status.
 int launch_cf_mid(const CFArgs &a, cudaStream_t s, cudaError_t *e);
 cudaError_t launch_cf_generic(const CFArgs &a, int warps, int grid, cudaStream_t s);
-cudaError_t launch_convert(const ConvProgram &pr, const PlanePtr *in_dev, const PlanePtr *out_dev,
-                           int nframes, cudaStream_t s);
+// in / out: host arrays of nframes * pr.nin / pr.nout planes (an output without an address is left out)
+cudaError_t launch_convert(const ConvProgram &pr, const PlanePtr *in, const PlanePtr *out, int nframes, cudaStream_t s);
 cudaError_t launch_finalize(const FinalizeArgs &a, int nframes, cudaStream_t s);
 cudaError_t launch_vaggregate(const VAggArgs &a, int nframes, cudaStream_t s);
 cudaError_t launch_vstack(const VStackArgs &a, int nframes, cudaStream_t s);
