@@ -1793,9 +1793,8 @@ private:
         for (int k = 0; k < count; ++k)
             for (int p = 0; p < 3; ++p) {
                 if (p < np && process[p]) {
-                    PlanePtr t = stager_.target(*dst[k], p, go);
-                    CU(cudaMemset2DAsync(t.ptr, t.stride, 0, (size_t)W * 4, ovi.height, stream));
-                    outs.push_back(t);
+                    // every slot is written, also the empty ones of a window cut off by the clip's ends
+                    outs.push_back(stager_.target(*dst[k], p, go));
                 } else {
                     outs.push_back(PlanePtr{nullptr, 0});
                 }
