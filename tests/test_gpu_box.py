@@ -88,3 +88,9 @@ def test_nan_stays_in_the_groups_that_hold_it(orc):
     src[0, 0, 30, 40] = np.nan
     check(orc, src, ref, th_mse=40.0)
     check(orc, src, None)
+
+
+def test_weights_of_huge_values(orc):
+    """Spectra whose squares leave the range of the reciprocal estimate (and, further on, of fp32)."""
+    src, ref = pair(40, 56)
+    check(orc, src * np.float32(1e15), ref * np.float32(1e15), th_mse=1e33)

@@ -19,7 +19,7 @@
 // Bound: the FP32 pipe (9.9 k clocks of a step's 19 k; the transforms are separable butterflies, and a
 // packed instruction takes the pipe twice) and, in the phases that do not use it, the latency of 16
 // warps per SM, which the transpose buffers and 128 registers a thread allow.  1920x1080 RGB x 8,
-// G = 32: 120.3 ms with one warp per group, gathers from global memory and a 64-bit box, 47.9 ms now.
+// G = 32: 120.3 ms with one warp per group, gathers from global memory and a 64-bit box, 44.1 ms now.
 #pragma once
 
 #include "cf.cuh"
@@ -162,31 +162,74 @@ __device__ __forceinline__ void idct_sets(const float (&X)[N], F &&f)
     }
 }
 
-// w[i] = r2[i] / (r2[i] + sg): reciprocal estimate, quotient, and one correction by the exact remainder
-// (Markstein, IBM J. Res. Dev. 34, 1990), which rounds as the division does but for quotients within a
-// few 2^-46 of a tie.  The division itself (a dozen instructions and a branch each) serves where the
-// estimate would underflow.
-template <int C>
-__device__ __forceinline__ void wiener_weights(const float (&r2)[C], float sg, float (&w)[C])
+// Wiener weights w[i] = r2[i] / (r2[i] + sg): reciprocal estimate, quotient, and one correction by the exact
+// remainder (Markstein, IBM J. Res. Dev. 34, 1990), which rounds as the division does but for quotients
+// within a few 2^-46 of a tie.  EXACT: the division itself, a dozen instructions and a branch each.  The estimate
+// underflows for divisors from 2^126 on: `top` collects the largest, and a column that has one is redone.
+constexpr float kWienerTop = 4.2535296e37f;       // 2^125
+
+template <bool EXACT, int C>
+__device__ __forceinline__ void wiener_weights(const float (&r2)[C], float sg, float (&w)[C], float &top)
 {
-    float d[C], top = 0.0f;
 #pragma unroll
     for (int i = 0; i < C; ++i) {
-        d[i] = __fadd_rn(r2[i], sg);
-        top = fmaxf(top, d[i]);
+        const float d = __fadd_rn(r2[i], sg);
+        if constexpr (EXACT) {
+            w[i] = __fdiv_rn(r2[i], d);
+        } else {
+            top = fmaxf(top, d);
+            float y;
+            asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(d));
+            const float q = __fmul_rn(r2[i], y);
+            w[i] = __fmaf_rn(__fmaf_rn(-d, q, r2[i]), y, q);
+        }
     }
-    if (top < 4.2535296e37f) {            // 2^125
+}
+
+// A column of N (reference, source) cells filtered by its Wiener weights: its spectrum in Y; returns the sum of
+// the squared weights
+template <int N, bool EXACT>
+__device__ __forceinline__ float wiener_spectrum(const f2 (&x)[N], float sg, float (&Y)[N], float &top)
+{
+    float l2 = 0.0f;
+    fdct2<N>(x, [&](int k, int st, const auto &v) {
+        constexpr int C = (int)(sizeof(v) / sizeof(v[0]));
+        float r2[C], sv[C], w[C];
 #pragma unroll
         for (int i = 0; i < C; ++i) {
-            float y;
-            asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(d[i]));
-            const float q = __fmul_rn(r2[i], y);
-            w[i] = __fmaf_rn(__fmaf_rn(-d[i], q, r2[i]), y, q);
+            float r;
+            upk(v[i], r, sv[i]);
+            r2[i] = __fmul_rn(r, r);
         }
-    } else {
+        wiener_weights<EXACT, C>(r2, sg, w, top);
 #pragma unroll
-        for (int i = 0; i < C; ++i) w[i] = __fdiv_rn(r2[i], d[i]);
-    }
+        for (int i = 0; i < C; ++i) {
+            Y[k + i * st] = __fmul_rn(sv[i], w[i]);
+            l2 = __fmaf_rn(w[i], w[i], l2);
+        }
+    });
+    return l2;
+}
+
+// Z stage of a column of N cells (stride in cells), the filtered source into the cells' low words
+template <int N, bool EXACT>
+__device__ __forceinline__ float wiener_column(f2 *t, int stride, float sg, float &top)
+{
+    f2 x[N];
+    float Y[N];
+#pragma unroll
+    for (int z = 0; z < N; ++z) x[z] = t[z * stride];
+    const float l2 = wiener_spectrum<N, EXACT>(x, sg, Y, top);
+    if (EXACT || top < kWienerTop) idct_sets<N>(Y, [&](int z, float v) { *reinterpret_cast<float *>(t + z * stride) = v; });
+    return l2;
+}
+
+// out of line: huge values only
+template <int N>
+__device__ __noinline__ float wiener_column_exact(f2 *t, int stride, float sg)
+{
+    float top = 0.0f;
+    return wiener_column<N, true>(t, stride, sg, top);
 }
 
 constexpr int kBT = 66;                  // cells between the blocks of the transpose buffer: 2 mod 16, so that
@@ -306,36 +349,16 @@ __device__ __forceinline__ void box_add(f2 v, int *c0, int *c1, int low)
     atomicAdd(c1 + low, __float_as_int(l1) - kBoxRoundBits);
 }
 
-// Wiener z stage of one coefficient column (cells t[z * kBT]) of a group of N blocks: the filtered source
-// column into the cells' low words; returns the sum of the squared weights
+// Wiener z stage of one coefficient column (cells t[z * kBT]) of a group of N blocks; returns the sum of the
+// squared weights
 template <int N>
 __device__ __noinline__ float box_wiener(int at, float sg)
 {
     extern __shared__ __align__(16) float smem[];
     f2 *t = reinterpret_cast<f2 *>(smem) + at;
-    f2 x[N];
-    float Y[N];
-#pragma unroll
-    for (int z = 0; z < N; ++z) x[z] = t[z * kBT];
-    float l2 = 0.0f;
-    fdct2<N>(x, [&](int k, int st, const auto &v) {
-        constexpr int C = (int)(sizeof(v) / sizeof(v[0]));
-        float r2[C], sv[C], w[C];
-#pragma unroll
-        for (int i = 0; i < C; ++i) {
-            float r;
-            upk(v[i], r, sv[i]);
-            r2[i] = __fmul_rn(r, r);
-        }
-        wiener_weights<C>(r2, sg, w);
-#pragma unroll
-        for (int i = 0; i < C; ++i) {
-            Y[k + i * st] = __fmul_rn(sv[i], w[i]);
-            l2 = __fmaf_rn(w[i], w[i], l2);
-        }
-    });
-    idct_sets<N>(Y, [&](int z, float v) { reinterpret_cast<float *>(t + z * kBT)[0] = v; });
-    return l2;
+    float top = 0.0f;
+    const float l2 = wiener_column<N, false>(t, kBT, sg, top);
+    return top < kWienerTop ? l2 : wiener_column_exact<N>(t, kBT, sg);
 }
 
 // the same for a length without an unrolled transform: the direct sums of both columns at once
@@ -497,10 +520,11 @@ __global__ void __launch_bounds__(NP * 64, 8 / NP) cf_box_kernel(CFArgs a, CFBox
         const float denW = __fdiv_rn(1.0f, l2 > eps ? l2 : eps);
         box_inverse(reinterpret_cast<float *>(tb), active ? __fdiv_rn(denW, a.amp[n - 1]) : 0.0f, active, h);
         __syncwarp();
-        // aggregation, four blocks per step
+        // aggregation, four blocks per step (not unrolled further: the step's code already overflows the
+        // instruction caches)
         const float *v = reinterpret_cast<const float *>(tr + pair * kT + 16 * role * kBT) + lane;
         int *cell = acc + sy * P + sx, *cell0 = acc + sy * 8 + sx;
-#pragma unroll
+#pragma unroll 1
         for (int i = 0; i < 16; i += 4) {
             f2 e[4];
             int o[4];

@@ -82,28 +82,9 @@ __device__ __forceinline__ void mid_transform(T *v, int stride, int B, const flo
 template <int N>
 __device__ __forceinline__ float mid_z(f2 *v, int stride, float sg, float)
 {
-    f2 x[N];
-    float Y[N], l2 = 0.0f;
-#pragma unroll
-    for (int z = 0; z < N; ++z) x[z] = v[z * stride];
-    fdct2<N>(x, [&](int k, int st, const auto &u) {
-        constexpr int C = (int)(sizeof(u) / sizeof(u[0]));
-        float r2[C], s[C], w[C];
-#pragma unroll
-        for (int i = 0; i < C; ++i) {
-            float r;
-            upk(u[i], r, s[i]);
-            r2[i] = __fmul_rn(r, r);
-        }
-        wiener_weights<C>(r2, sg, w);
-#pragma unroll
-        for (int i = 0; i < C; ++i) {
-            Y[k + i * st] = __fmul_rn(s[i], w[i]);
-            l2 = __fmaf_rn(w[i], w[i], l2);
-        }
-    });
-    idct_sets<N>(Y, [&](int z, float u) { *reinterpret_cast<float *>(v + z * stride) = u; });
-    return l2;
+    float top = 0.0f;
+    const float l2 = wiener_column<N, false>(v, stride, sg, top);
+    return top < kWienerTop ? l2 : wiener_column_exact<N>(v, stride, sg);
 }
 
 template <int N>
