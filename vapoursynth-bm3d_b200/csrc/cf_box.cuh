@@ -649,6 +649,24 @@ __device__ __noinline__ int box_hard_any(int at, int half, float t0, float t1, i
     return kept;
 }
 
+// z stage of the two groups at a column, of ma and mb blocks (0: no group): the warp's kept counts in the halves
+// of an int.  Groups of the same full length go together, others one by one.
+template <int G>
+__device__ __forceinline__ int box_hard_pair(int at, const CFArgs &a, int p, int fxy, int ma, int mb)
+{
+    int kept = 0;
+    if (ma == G && mb == G) kept = box_hard<G>(at, a.thr4[p][G - 1][fxy + 1], a.thr4[p][G - 1][fxy]);
+    else {
+#pragma unroll 1
+        for (int half = 0; half < 2; ++half) {
+            const int m = half ? mb : ma, i = max(m, 1) - 1;
+            kept += box_hard_any(at, half, a.thr4[p][i][fxy + 1], a.thr4[p][i][fxy], m, dtab_for(a, m, false),
+                                 dtab_for(a, m, true)) << (16 * half);
+        }
+    }
+    return __reduce_add_sync(0xffffffffu, kept);
+}
+
 // Inverse 2-D transform of both halves of the cells at `t`, scaled, in place: pixel (y, x) to cell 8 x + y.
 // Lane half h inverts the columns 2k + h, then the rows 2i + h.
 __device__ __forceinline__ void box_inverse2(f2 *t, f2 scale, bool activeA, bool activeB, int h)
@@ -772,19 +790,7 @@ __global__ void __launch_bounds__(NP * 64, 8 / NP) cf_boxh_kernel(CFArgs a, CFBo
         for (int q = 0; q < GPW; ++q) {
             const int ma = q < gA ? min(a.count[grpA + q], G) : 0, mb = q < gB ? min(a.count[grpB + q], G) : 0;
             const int at = pair * kT + q * G * kBT + col;
-            int kept;
-            // groups of the same full length together, others one by one
-            if (ma == G && mb == G) kept = box_hard<G>(at, a.thr4[p][G - 1][fxy + 1], a.thr4[p][G - 1][fxy]);
-            else {
-                kept = 0;
-#pragma unroll 1
-                for (int half = 0; half < 2; ++half) {
-                    const int m = half ? mb : ma, i = max(m, 1) - 1;
-                    kept += box_hard_any(at, half, a.thr4[p][i][fxy + 1], a.thr4[p][i][fxy], m, dtab_for(a, m, false),
-                                         dtab_for(a, m, true)) << (16 * half);
-                }
-            }
-            kept = __reduce_add_sync(0xffffffffu, kept);
+            const int kept = box_hard_pair<G>(at, a, p, fxy, ma, mb);
             if (lane == 0) red[2 * q + role] = kept;
         }
         pair_barrier(1 + pair);
@@ -851,6 +857,183 @@ __global__ void __launch_bounds__(NP * 64, 8 / NP) cf_boxh_kernel(CFArgs a, CFBo
 
     __syncthreads();
     box_flush(acc, cells, slot0, P, a.num[p] + f * a.frame_stride, a.ld, y0, x0, bh, bw);
+}
+
+// ---- V-BM3D: the same warp pairs without a box -----------------------------------------------------------
+// A group's blocks lie in up to 2 radius + 1 frames, so there is no box to stage: blocks are read from and added to
+// the planes one per warp step (lane = row and column of half a block), through the transpose buffer.
+// Bound: latency of the steps and the L2's atomics.  1280x720 YUV x 7, radius 3, Final, G = 8: 7.4 ms
+// with per-lane gathers and atomics (cf_fast_kernel), 4.8 ms here.
+
+// offsets of the lane's block in the source planes and in the accumulators (locate() with 64-bit offsets)
+__device__ __forceinline__ void pair_locate(const CFArgs &a, long long grp, uint32_t pk, long long &src, long long &acc)
+{
+    const long long f = grp / a.blocks_per_frame;
+    if (!a.vbm3d) {
+        src = acc = f * a.frame_stride + (long long)unpack_y(pk) * a.ld + unpack_x(pk);
+    } else {
+        const int z = unpack3_z(pk);
+        const long long at = (long long)unpack3_y(pk) * a.ld + unpack3_x(pk);
+        src = ((long long)a.win_base[f] + z) * a.frame_stride + at;
+        acc = (f * a.slots + a.slot0[f] + z) * a.acc_stride + at;
+    }
+}
+
+template <int G, int NP>
+__global__ void __launch_bounds__(NP * 64, 8 / NP) cf_pair_kernel(const __grid_constant__ CFArgs a)
+{
+    extern __shared__ __align__(16) float smem[];
+    constexpr int GPW = 32 / G, kT = 32 * kBT;
+    const int lane = (int)lane_id();
+    const int warp = threadIdx.x >> 5, pair = warp >> 1, role = warp & 1;
+    f2 *tr = reinterpret_cast<f2 *>(smem) + pair * kT;
+    float *red = smem + 2 * NP * kT + pair * 2 * GPW;
+    const int h = lane & 1, blk = 16 * role + (lane >> 1), sub = blk / G, z = blk - sub * G;
+    f2 *tb = tr + blk * kBT, *tw = tr + 16 * role * kBT;
+    const int ry = lane >> 3, cx = lane & 7;
+    const long long nslots = (a.ngroups + GPW - 1) / GPW;
+    for (long long slot = (long long)blockIdx.x * NP + pair; slot < nslots; slot += (long long)gridDim.x * NP) {
+        const long long grp = slot * GPW + sub;
+        const int n = grp < a.ngroups ? min(a.count[grp], G) : 0;
+        const bool active = z < n;
+        long long so = 0, ao = 0;
+        if (active) pair_locate(a, grp, a.pos[grp * G + z], so, ao);
+        for (int p = 0; p < 3; ++p) {
+            if (!a.process[p]) continue;
+            const float *src = a.src[p], *ref = a.ref[p];
+            __syncwarp();
+#pragma unroll 4
+            for (int i = 0; i < 16; ++i) {
+                const long long o = __shfl_sync(0xffffffffu, so, 2 * i) + (long long)ry * a.ld + cx;
+                tw[i * kBT + lane] = pk(__ldg(ref + o), __ldg(src + o));
+                tw[i * kBT + 32 + lane] = pk(__ldg(ref + o + 4ll * a.ld), __ldg(src + o + 4ll * a.ld));
+            }
+            __syncwarp();
+            {
+                f2 x[4][8];
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+#pragma unroll
+                    for (int k = 0; k < 8; ++k) x[i][k] = tb[(h ? 7 - i : i) * 8 + k];
+                __syncwarp();
+                box_forward([&](int i, int k) { return x[i][k]; }, tb, h);
+            }
+            pair_barrier(1 + pair);
+#pragma unroll 1
+            for (int q = 0; q < GPW; ++q) {
+                if (slot * GPW + q >= a.ngroups) break;
+                const int nq = min(a.count[slot * GPW + q], G);
+                float l2 = box_wiener_any<G>(pair * kT + q * G * kBT + role * 32 + lane, a.wsig2[p][nq - 1], nq, a);
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1) l2 = __fadd_rn(l2, __shfl_xor_sync(0xffffffffu, l2, o));
+                if (lane == 0) red[2 * q + role] = l2;
+            }
+            pair_barrier(1 + pair);
+            const float l2 = __fadd_rn(red[2 * sub], red[2 * sub + 1]);
+            const float eps = 1.1920928955078125e-07f;
+            const float denW = __fdiv_rn(1.0f, l2 > eps ? l2 : eps);
+            box_inverse(reinterpret_cast<float *>(tb), active ? __fdiv_rn(denW, a.amp[n - 1]) : 0.0f, active, h);
+            __syncwarp();
+            const unsigned mask = __ballot_sync(0xffffffffu, active);
+            float *num = a.num[p];
+#pragma unroll 4
+            for (int i = 0; i < 16; ++i) {
+                const long long o = __shfl_sync(0xffffffffu, ao, 2 * i) + (long long)ry * a.ld + cx;
+                const float *v = reinterpret_cast<const float *>(tw + i * kBT) + cx * 8 + ry;
+                if (mask >> (2 * i) & 1) {
+                    atomicAdd(num + o, v[0]);
+                    atomicAdd(num + o + 4ll * a.ld, v[4]);
+                }
+            }
+            if (active && h == 0) atomicAdd(a.wmap[p] + ao, denW);
+        }
+    }
+}
+
+template <int G, int NP>
+__global__ void __launch_bounds__(NP * 64, 8 / NP) cf_pairh_kernel(const __grid_constant__ CFArgs a)
+{
+    extern __shared__ __align__(16) float smem[];
+    constexpr int GPW = 32 / G, kT = 32 * kBT;
+    const int lane = (int)lane_id();
+    const int warp = threadIdx.x >> 5, pair = warp >> 1, role = warp & 1;
+    f2 *tr = reinterpret_cast<f2 *>(smem) + pair * kT;
+    int *red = reinterpret_cast<int *>(smem + 2 * NP * kT) + pair * 2 * GPW;
+    const int h = lane & 1, blk = 16 * role + (lane >> 1), sub = blk / G, z = blk - sub * G;
+    f2 *tb = tr + blk * kBT, *tw = tr + 16 * role * kBT;
+    const int ry = lane >> 3, cx = lane & 7;
+    const int col = role * 32 + lane, fxy = ((col & 7) == 0) + ((col >> 3) == 0);
+    const long long nslots = (a.ngroups + GPW - 1) / GPW;
+    for (long long slot = 2 * ((long long)blockIdx.x * NP + pair); slot < nslots; slot += 2ll * gridDim.x * NP) {
+        const long long gA = slot * GPW + sub, gB = gA + GPW;
+        const int na = gA < a.ngroups ? min(a.count[gA], G) : 0, nb = gB < a.ngroups ? min(a.count[gB], G) : 0;
+        const bool actA = z < na, actB = z < nb;
+        long long sA = 0, oA = 0, sB = 0, oB = 0;
+        if (actA) pair_locate(a, gA, a.pos[gA * G + z], sA, oA);
+        if (actB) pair_locate(a, gB, a.pos[gB * G + z], sB, oB);
+        for (int p = 0; p < 3; ++p) {
+            if (!a.process[p]) continue;
+            const float *src = a.src[p];
+            __syncwarp();
+#pragma unroll 4
+            for (int i = 0; i < 16; ++i) {
+                const long long u = __shfl_sync(0xffffffffu, sA, 2 * i) + (long long)ry * a.ld + cx;
+                const long long v = __shfl_sync(0xffffffffu, sB, 2 * i) + (long long)ry * a.ld + cx;
+                tw[i * kBT + lane] = pk(__ldg(src + u), __ldg(src + v));
+                tw[i * kBT + 32 + lane] = pk(__ldg(src + u + 4ll * a.ld), __ldg(src + v + 4ll * a.ld));
+            }
+            __syncwarp();
+            {
+                f2 x[4][8];
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+#pragma unroll
+                    for (int k = 0; k < 8; ++k) x[i][k] = tb[(h ? 7 - i : i) * 8 + k];
+                __syncwarp();
+                box_forward([&](int i, int k) { return x[i][k]; }, tb, h);
+            }
+            pair_barrier(1 + pair);
+#pragma unroll 1
+            for (int q = 0; q < GPW; ++q) {
+                const long long ga = slot * GPW + q, gb = ga + GPW;
+                const int ma = ga < a.ngroups ? min(a.count[ga], G) : 0, mb = gb < a.ngroups ? min(a.count[gb], G) : 0;
+                const int kept = box_hard_pair<G>(pair * kT + q * G * kBT + col, a, p, fxy, ma, mb);
+                if (lane == 0) red[2 * q + role] = kept;
+            }
+            pair_barrier(1 + pair);
+            const int kept = red[2 * sub] + red[2 * sub + 1], kA = kept & 0xffff, kB = kept >> 16;
+            if (a.retained && z == 0 && h == 0) {
+                if (na) a.retained[(long long)p * a.ngroups + gA] = kA;
+                if (nb) a.retained[(long long)p * a.ngroups + gB] = kB;
+            }
+            const float dA = kA < 1 ? 1.0f : __fdiv_rn(1.0f, (float)kA), dB = kB < 1 ? 1.0f : __fdiv_rn(1.0f, (float)kB);
+            box_inverse2(tb, pk(actA ? __fdiv_rn(dA, a.amp[na - 1]) : 0.0f, actB ? __fdiv_rn(dB, a.amp[nb - 1]) : 0.0f), actA, actB, h);
+            __syncwarp();
+            const unsigned mA = __ballot_sync(0xffffffffu, actA), mB = __ballot_sync(0xffffffffu, actB);
+            float *num = a.num[p];
+#pragma unroll 4
+            for (int i = 0; i < 16; ++i) {
+                const long long u = __shfl_sync(0xffffffffu, oA, 2 * i) + (long long)ry * a.ld + cx;
+                const long long v = __shfl_sync(0xffffffffu, oB, 2 * i) + (long long)ry * a.ld + cx;
+                const f2 *e = tw + i * kBT + cx * 8 + ry;
+                float a0, b0, a1, b1;
+                upk(e[0], a0, b0);
+                upk(e[4], a1, b1);
+                if (mA >> (2 * i) & 1) {
+                    atomicAdd(num + u, a0);
+                    atomicAdd(num + u + 4ll * a.ld, a1);
+                }
+                if (mB >> (2 * i) & 1) {
+                    atomicAdd(num + v, b0);
+                    atomicAdd(num + v + 4ll * a.ld, b1);
+                }
+            }
+            if (h == 0) {
+                if (actA) atomicAdd(a.wmap[p] + oA, dA);
+                if (actB) atomicAdd(a.wmap[p] + oB, dB);
+            }
+        }
+    }
 }
 
 }  // namespace bm3d

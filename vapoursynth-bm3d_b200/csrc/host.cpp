@@ -1298,7 +1298,11 @@ public:
                 return;
             }
         }
-        // kernels that leave counts out (the box form writes every processed plane's)
+        if (fast && !tensor) {
+            CU(launch_cf_pair(a, stream));
+            return;
+        }
+        // kernels that leave counts out (the forms above write every processed plane's)
         if (!wiener) CU(cudaMemsetAsync(a.retained, 0xff, sizeof(int) * 3 * (size_t)std::max<long long>(1, ngroups), stream));
         if (tensor) {
             a.recheck_band = recheck_band;

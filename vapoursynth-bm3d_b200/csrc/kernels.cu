@@ -244,6 +244,30 @@ int launch_cf_box(const CFArgs &a, const CFBox &g, int step, cudaStream_t s, cud
     }
 }
 
+template <int G>
+static cudaError_t launch_cf_pair_t(const CFArgs &a, cudaStream_t s)
+{
+    constexpr int NP = 4;
+    auto kernel = a.wiener ? cf_pair_kernel<G, NP> : cf_pairh_kernel<G, NP>;
+    const size_t smem = (size_t)NP * 32 * kBT * 8 + (size_t)NP * 2 * (32 / G) * 4;
+    cudaError_t e;
+    if ((e = allow_smem(kernel, smem)) != cudaSuccess) return e;
+    const long long per = (long long)NP * (32 / G) * (a.wiener ? 1 : 2);       // groups of a CTA's step
+    COUNT_LAUNCH();
+    kernel<<<(unsigned)std::max<long long>(1, std::min<long long>((a.ngroups + per - 1) / per, 148LL * 8)), NP * 64, smem, s>>>(a);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_cf_pair(const CFArgs &a, cudaStream_t s)
+{
+    switch (a.B == 8 ? a.G : 0) {
+    case 8: return launch_cf_pair_t<8>(a, s);
+    case 16: return launch_cf_pair_t<16>(a, s);
+    case 32: return launch_cf_pair_t<32>(a, s);
+    default: return cudaErrorInvalidValue;
+    }
+}
+
 template <int G, bool W>
 static cudaError_t launch_cf_fast_t(const CFArgs &a, cudaStream_t s)
 {

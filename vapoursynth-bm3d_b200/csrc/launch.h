@@ -36,6 +36,9 @@ cudaError_t launch_vbm_predict(const VBMArgs &a, bool fast, int nframes, size_t 
 // Plain Final filter of BM3D frames (B = 8, G in {8, 16, 32}) with a run's image region in shared
 // memory; returns 0 if the shape is not its own or the region does not fit, else 1 and the status.
 int launch_cf_box(const CFArgs &a, const CFBox &g, int step, cudaStream_t s, cudaError_t *e);
+// The same warp pairs without a staged region: V-BM3D groups, and regions too large to stage (B = 8, G in
+// {8, 16, 32}).
+cudaError_t launch_cf_pair(const CFArgs &a, cudaStream_t s);
 // Fast collaborative filter (B = 8, G in {8, 16, 32}, any group length n <= G); sizes its own
 // grid; returns cudaErrorInvalidValue for other shapes.
 cudaError_t launch_cf_fast(const CFArgs &a, cudaStream_t s);
