@@ -41,8 +41,15 @@ BM3D_HD inline int vbm_warp_floats(int sp_cap, int list_cap, int G, int ps_num, 
 
 // vbm_predict8_kernel: the window of a centre (2 range + 8 rows and columns) fits a warp's 32 lanes
 constexpr int kPsMaxRange = 12;
-BM3D_HD inline int vbm8_pitch(int range) { return 2 * range + 9; }   // odd: lanes on consecutive rows
-BM3D_HD inline int vbm8_patch_floats(int range) { return ((2 * range + 8) * vbm8_pitch(range) + 7) & ~3; }
+// a centre's window as pairs of rows, those that start at an even row and then those at an odd one; lanes on
+// consecutive rows read them in turn: odd pitch, and 8 mod 16 pairs between the two sets
+BM3D_HD inline int vbm8_pitch(int range) { return 2 * range + 9; }
+BM3D_HD inline int vbm8_odd(int range)
+{
+    const int n = (range + 4) * vbm8_pitch(range);
+    return n + (24 - n % 16) % 16;
+}
+BM3D_HD inline int vbm8_patch_floats(int range) { return 2 * ((vbm8_odd(range) + (range + 3) * vbm8_pitch(range) + 5) & ~1); }
 // per warp: a work region -- two window patches and the lanes' distances (four candidates per lane
 // and round), or sp, tmp and sk of a search redone by the general routines, or the keys of the
 // concatenated list in lane columns ...
@@ -54,10 +61,10 @@ BM3D_HD inline int vbm8_work_floats(int range, int sp_cap, int list_cap)
     if (n < list_cap + 32) n = list_cap + 32;
     return (n + 3) & ~3;
 }
-// ... after the reference block; then the list (keys, positions), a frame's selection, two centres
+// ... after the reference block, by rows and by pairs of rows; then the list (keys, positions), a frame's selection, two centres
 BM3D_HD inline int vbm8_warp_floats(int range, int sp_cap, int list_cap, int G)
 {
-    return (64 + vbm8_work_floats(range, sp_cap, list_cap) + 2 * list_cap + 2 * G + 2 + 3) & ~3;
+    return (128 + vbm8_work_floats(range, sp_cap, list_cap) + 2 * list_cap + 2 * G + 2 + 3) & ~3;
 }
 
 // bm_est_kernel: window pitch in row pairs, place of the pairs that start at odd rows, pairs in all,

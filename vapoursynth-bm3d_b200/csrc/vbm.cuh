@@ -354,8 +354,9 @@ __global__ void __launch_bounds__(128) vbm_predict_kernel(VBMArgs a)
 // union only decides between equal keys: a search whose kept keys, or the key at the cut, are not
 // distinct is redone by the general routines.
 // Bound: FP32 issue of the distances.  1280x720 x 7 frames, radius 3, 169 to 338 candidates per
-// search: predictive search 77.9 ms before, 15.0 ms now; 1920x1080 x 5 frames, radius 1,
-// 81 to 162 candidates: 4.74 -> 1.10 ms.
+// search: predictive search 77.9 ms before, 13.5 ms now; 1920x1080 x 5 frames, radius 1,
+// 81 to 162 candidates: 4.74 -> 1.02 ms.  (With windows by rows, whose packed pairs of columns have to be
+// re-packed by moves for every other candidate: 15.0 and 1.10 ms.)
 
 // Exact distances and the reference's selection over one frame's union: keys and positions of the
 // frame's list into fk / fp; returns its length.
@@ -430,7 +431,7 @@ __device__ __forceinline__ int warp_smallest(LaneBest &lb, float *col, int nslot
     return n;
 }
 
-__global__ void __launch_bounds__(128) vbm_predict8_kernel(VBMArgs a)
+__global__ void __launch_bounds__(128, 5) vbm_predict8_kernel(VBMArgs a)
 {
     extern __shared__ __align__(16) float smem[];
     const int lane = (int)lane_id();
@@ -443,8 +444,10 @@ __global__ void __launch_bounds__(128) vbm_predict8_kernel(VBMArgs a)
     const int R = a.ps_range, G = a.G;
     const int P = vbm8_pitch(R);
     float *rblk = smem + (size_t)warp * vbm8_warp_floats(R, a.sp_cap, a.list_cap, G);
-    float *work = rblk + 64;
-    float *patch0 = work, *patch1 = work + vbm8_patch_floats(R);
+    f32x2 *rpair = reinterpret_cast<f32x2 *>(rblk + 64);
+    float *work = rblk + 128;
+    f32x2 *patch0 = reinterpret_cast<f32x2 *>(work), *patch1 = reinterpret_cast<f32x2 *>(work + vbm8_patch_floats(R));
+    const int odd = vbm8_odd(R);
     float *col = work + 2 * vbm8_patch_floats(R) + lane;
     float *lk = work + vbm8_work_floats(R, a.sp_cap, a.list_cap);
     uint32_t *lp = reinterpret_cast<uint32_t *>(lk + a.list_cap);
@@ -478,8 +481,25 @@ __global__ void __launch_bounds__(128) vbm_predict8_kernel(VBMArgs a)
 #pragma unroll
     for (int e = 0; e < 64; e += 32) {
         const int idx = e + lane;
-        rblk[idx] = curplane[(long long)(j + (idx >> 3)) * a.ld + i + (idx & 7)];
+        const float v = curplane[(long long)(j + (idx >> 3)) * a.ld + i + (idx & 7)];
+        rblk[idx] = v;
+        reinterpret_cast<float *>(rpair + (idx >> 4) * 8 + (idx & 7))[(idx >> 3) & 1] = v;
     }
+    // window rows [t, t + rows), columns l .. l + cols - 1 of a plane to a patch, twice: as pairs of rows from even
+    // and from odd ones
+    auto stage = [&](f32x2 *patch, const float *plane, int t, int l, int rows, int cols) {
+        if (lane >= cols) return;
+        const float *src = plane + (long long)t * a.ld + l + lane;
+        float *e = reinterpret_cast<float *>(patch + lane), *o = reinterpret_cast<float *>(patch + odd + lane);
+        // rows 2q and 2q + 1: the halves of even pair q; the second half of odd pair q - 1 and the first of pair q
+        // (the last window row starts no pair)
+        for (int q = 0; 2 * q < rows; ++q, src += 2 * a.ld, e += 2 * P, o += 2 * P) {
+            tc::cp_async4(e, src);
+            if (q > 0) tc::cp_async4(o - 2 * P + 1, src);
+            if (2 * q + 1 < rows) tc::cp_async4(e + 1, src + a.ld);
+            if (2 * q + 2 < rows) tc::cp_async4(o, src + a.ld);
+        }
+    };
 
     const int ncen0 = min(a.ps_num, n0);
     for (int dir = -1; dir <= 1; dir += 2) {
@@ -492,14 +512,12 @@ __global__ void __launch_bounds__(128) vbm_predict8_kernel(VBMArgs a)
             const int t0 = max(0, y0 - R), b0 = min(a.H - 8, y0 + R), l0 = max(0, x0 - R), r0 = min(a.W - 8, x0 + R);
             const int t1 = max(0, y1 - R), b1 = min(a.H - 8, y1 + R), l1 = max(0, x1 - R), r1 = min(a.W - 8, x1 + R);
             __syncwarp();
-            for (int yy = 0; yy < b0 - t0 + 8; ++yy)
-                if (lane < r0 - l0 + 8) tc::cp_async4(patch0 + yy * P + lane, plane + (long long)(t0 + yy) * a.ld + l0 + lane);
+            stage(patch0, plane, t0, l0, b0 - t0 + 8, r0 - l0 + 8);
             // centre 1's candidates outside centre 0's window: rows [at, at + an) whole, rows
             // [it, it + in) of both windows in the columns [bl, bl + bn) only
             int at = t1, an = 0, it = 0, in = 0, bl = l1, bn = 0;
             if (ncen > 1) {
-                for (int yy = 0; yy < b1 - t1 + 8; ++yy)
-                    if (lane < r1 - l1 + 8) tc::cp_async4(patch1 + yy * P + lane, plane + (long long)(t1 + yy) * a.ld + l1 + lane);
+                stage(patch1, plane, t1, l1, b1 - t1 + 8, r1 - l1 + 8);
                 if (t1 > b0 || b1 < t0) an = b1 - t1 + 1;
                 else if (y1 >= y0) {          // the clamped windows keep the centres' order
                     it = t1; in = min(b0, b1) - t1 + 1;
@@ -517,13 +535,14 @@ __global__ void __launch_bounds__(128) vbm_predict8_kernel(VBMArgs a)
             const int nr0 = b0 - t0 + 1, nc0 = r0 - l0 + 1, nc1 = r1 - l1 + 1;
             const int i0 = nr0 * ((nc0 + 3) >> 2), iA = i0 + an * ((nc1 + 3) >> 2), items = iA + in * ((bn + 3) >> 2);
             // item -> first position of its four candidates, how many there are, and its patch
-            auto decode = [&](int item, int &y, int &x, int &nv) -> const float * {
+            auto at_row = [&](const f32x2 *patch, int r) { return patch + (r & 1 ? odd : 0) + (r >> 1) * P; };
+            auto decode = [&](int item, int &y, int &x, int &nv) -> const f32x2 * {
                 if (item < i0) {
                     const int q = item / nr0;
                     y = t0 + item - q * nr0;
                     x = l0 + 4 * q;
                     nv = nc0 - 4 * q;
-                    return patch0 + (y - t0) * P + (x - l0);
+                    return at_row(patch0, y - t0) + (x - l0);
                 }
                 if (item < iA) {
                     const int e = item - i0, q = e / an;
@@ -536,7 +555,7 @@ __global__ void __launch_bounds__(128) vbm_predict8_kernel(VBMArgs a)
                     x = bl + 4 * q;
                     nv = bn - 4 * q;
                 }
-                return patch1 + (y - t1) * P + (x - l1);
+                return at_row(patch1, y - t1) + (x - l1);
             };
             LaneBest lb;
             lb.clear();
@@ -544,32 +563,37 @@ __global__ void __launch_bounds__(128) vbm_predict8_kernel(VBMArgs a)
             for (int base = 0; base < items; base += 32, nslots += 4) {
                 const int item = base + lane;
                 int y = 0, x = 0, nv = 0;
-                const float *w0 = patch0;
+                const f32x2 *w0 = patch0;
                 if (item < items) w0 = decode(item, y, x, nv);
                 float acc[4][4];
 #pragma unroll
                 for (int u = 0; u < 4; ++u)
 #pragma unroll
                     for (int k = 0; k < 4; ++k) acc[u][k] = 0.0f;
+                // pairs of rows: difference and square packed, then each row's columns k and 4 + k into lane sum k
 #pragma unroll
-                for (int yy = 0; yy < 8; ++yy) {
-                    float w[11];
+                for (int yy = 0; yy < 4; ++yy) {
+                    f32x2 w[11], r[8];
 #pragma unroll
                     for (int k = 0; k < 11; ++k) w[k] = w0[yy * P + k];
-                    const ulonglong2 ra = *reinterpret_cast<const ulonglong2 *>(rblk + yy * 8);
-                    const ulonglong2 rb = *reinterpret_cast<const ulonglong2 *>(rblk + yy * 8 + 4);
-                    const f32x2 rp[4] = {ra.x, ra.y, rb.x, rb.y};
-                    f32x2 E[5], O[5];
 #pragma unroll
-                    for (int m = 0; m < 5; ++m) {
-                        E[m] = pack2(w[2 * m], w[2 * m + 1]);
-                        O[m] = pack2(w[2 * m + 1], w[2 * m + 2]);
+                    for (int k = 0; k < 8; k += 2) {
+                        const ulonglong2 q = *reinterpret_cast<const ulonglong2 *>(rpair + yy * 8 + k);
+                        r[k] = q.x;
+                        r[k + 1] = q.y;
                     }
 #pragma unroll
                     for (int u = 0; u < 4; ++u) {
-                        const f32x2 *Wp = (u & 1) ? O : E;
+                        float lo[8], hi[8];
 #pragma unroll
-                        for (int h = 0; h < 4; ++h) add_sq2(acc[u], h & 1, sub2(rp[h], Wp[(u >> 1) + h]));
+                        for (int k = 0; k < 8; ++k) {
+                            const f32x2 v = sub2(r[k], w[u + k]);
+                            unpack2(mul2(v, v), lo[k], hi[k]);
+                        }
+#pragma unroll
+                        for (int k = 0; k < 4; ++k) acc[u][k] = __fadd_rn(__fadd_rn(acc[u][k], lo[k]), lo[4 + k]);
+#pragma unroll
+                        for (int k = 0; k < 4; ++k) acc[u][k] = __fadd_rn(__fadd_rn(acc[u][k], hi[k]), hi[4 + k]);
                     }
                 }
 #pragma unroll
