@@ -6,10 +6,8 @@ Workload (one step): 8 synthetic RGB float32 1920x1080 frames per GPU through
     matrix=100) -> OPP2RGB(sample=1), sigma 10,
 the full-pipeline configuration of the reference plugin's benchmark (8 frames, 1080p RGB).
 Four forms run: the plain FP32 path (precision="fp32", the oracle-exact drop-in), the precision
-form (precision="tf32": tensor-core transforms, tensor-core matching estimates with exact
-re-rank), the same with Basic at precision="tf32_match" ("tf32_final": Basic's matching on the
-tensor cores but its hard-threshold filter on the plain transform, the Final filter on the tensor
-cores) and the learned-proposal form
+form (precision="tf32": tensor-core transforms), the same with Basic at precision="tf32_match"
+("tf32_final": Basic on the plain transform, the Final filter on the tensor cores) and the learned-proposal form
 (precision="learned": as tf32, but matching re-ranks only the proposals of the learned descriptor
 network).  `value` is the fastest of the tensor-core forms whose output PSNR against the clean
 frames stays within 0.05 dB of the plain path's (else the plain path's); `forms` gives all four.  `value` times the device-resident pipeline (frames

@@ -188,10 +188,9 @@ BM3D_API int bm3d_debug_reference_fp64(bm3d_filter *filter, int k, double *plane
 BM3D_API int64_t bm3d_debug_launch_count(void);
 /* Number of reference blocks that took the exact tie-resolution path in the last call. */
 BM3D_API int64_t bm3d_debug_slow_blocks(bm3d_filter *filter);
-/* Precision form ("tf32") block matching of the last call: reference blocks whose tensor-core
- * distance estimates could not settle the list (all distances then computed exactly), and CTAs
- * whose tensor-core wait timed out (their blocks also computed exactly).  No reference
- * counterpart.  Returns 0, or -1 for a null filter. */
+/* Full-search block matching of the last call: reference blocks whose distance estimates could not
+ * settle the list (all distances then computed exactly); timeouts is always 0 (kept from a
+ * tensor-core form of the estimates).  No reference counterpart.  Returns 0, or -1 for a null filter. */
 BM3D_API int bm3d_debug_bm_tc_counts(bm3d_filter *filter, int64_t *fallbacks, int64_t *timeouts);
 /* Precision form ("tf32"), hard threshold (Basic / VBasic), last call: coefficients whose
  * tensor-core value lay within the recheck band of their threshold and were recomputed in fp32,

@@ -757,8 +757,8 @@ class BM3DBase : public Filter {
 public:
     bool wiener = false;
     bool vbm3d = false;
-    bool tc = false;            // precision form: tensor-core matching estimates (argument "precision")
-    bool tc_cf = false;         // precision form: tensor-core transforms as well
+    bool tc = false;            // argument "precision" other than "fp32"
+    bool tc_cf = false;         // precision form: tensor-core transforms
     bool learned = false;       // precision "learned": block matching by learned proposals
     // extension of VBasic / VFinal: aggregate = 1 returns VAggregate(radius, sample) of the
     // filter's output directly, without the stacked clip
@@ -1139,7 +1139,7 @@ public:
 
     void ensure_ws(int nslots, int nout)
     {
-        for (int p = 0; p < 3; ++p) {
+        for (int p = 0; p < nplanes(); ++p) {
             ws_src[p].get(sizeof(float) * fs * nslots);
             if (rdef) ws_ref[p].get(sizeof(float) * fs * nslots);
         }
