@@ -308,8 +308,8 @@ def ours_arm(args):
     stream = torch.cuda.Stream()
     vi = capi.VideoInfo(capi.RGB, capi.FLOAT, 32, 0, 0, Wd, Hd, F)
     # forms: the plain drop-in; tensor cores in both filters; the hard-threshold filter in FP32
-    # (exact decisions, and faster than its tensor-core version) after tensor-core matching, with
-    # the tensor-core Final; and the learned proposals
+    # (exact decisions, and faster than its tensor-core version) with the tensor-core Final; and
+    # the learned proposals
     precisions = {"fp32": "fp32", "tf32": "tf32", "tf32_final": ("tf32_match", "tf32"), "learned": "learned"}
     pipes = {form: Pipeline(L, capi, vi, stream, pr) for form, pr in precisions.items()}
 

@@ -893,8 +893,8 @@ public:
                 return fail(BM3D_ERR_ARG, err("Invalid \"hard_thr\" assigned, must be a positive floating point number"));
         }
         // extension: "precision" selects the plain FP32 path ("fp32", default), the tensor-core
-        // precision form ("tf32"), its matching alone with the plain transforms ("tf32_match":
-        // the same lists, so the output of "fp32") or the learned proposals ("learned")
+        // precision form ("tf32"), the plain path by another name ("tf32_match": it has
+        // the matching and the transforms of "fp32") or the learned proposals ("learned")
         const char *prec = map_get_data(in, "precision", 0, &error);
         if (!error) {
             const std::string pr(prec);
