@@ -33,6 +33,9 @@ namespace bm3d {
 constexpr float kEstEps = 1.52587890625e-5f;    // 2^-16
 constexpr int kEstCtas = 5;                     // CTAs per SM: 96 registers a thread, 41 KB at range 16
 constexpr float kEstTiny = 1e-30f;              // below it a distance may round to zero (never a match)
+// Largest threshold of this form.  A larger one is infinite in fp32, or nearly: then an infinite distance is a
+// match, which the empty slots of the estimates could not be told from, and the exact search takes the call.
+constexpr float kEstMaxThr = 1e38f;
 
 __device__ __forceinline__ f32x2 fma2_(f32x2 a, f32x2 b, f32x2 c)
 {
@@ -247,7 +250,8 @@ __global__ void __launch_bounds__(128, kEstCtas) bm_est_kernel(BMArgs a, EstLayo
     uint32_t *opos = a.out_pos + ob * G;
     float *okey = a.out_key ? a.out_key + ob * G : nullptr;
 
-    // the K + 1 smallest estimates among the surely valid, out of each lane's two smallest: an upper
+    // The threshold is finite with its margin (kEstMaxThr), so an empty slot, which is infinite, passes no test
+    // below.  The K + 1 smallest estimates among the surely valid, out of each lane's two smallest: an upper
     // bound on the K + 1 smallest distances.  Lane l takes element (l + 7 k) mod 32 of round k, so
     // that a compact patch of good candidates is spread over the lanes.
     const float ths = a.thSSE * (1.0f - 2.0f * kEstEps);
@@ -274,7 +278,7 @@ __global__ void __launch_bounds__(128, kEstCtas) bm_est_kernel(BMArgs a, EstLayo
         cut = __shfl_sync(0xffffffffu, v2[0], K);
     }
     const float bnd = fminf(a.thSSE, cut * (1.0f + 2.0f * kEstEps));      // on the exact distances
-    const float bt = complete ? thsure : cut * (1.0f + 4.0f * kEstEps);   // on the estimates
+    const float bt = fminf(thsure, cut * (1.0f + 4.0f * kEstEps));        // on the estimates
     // the band: every lane's own hits (at most kHits are kept), then one after the other
     constexpr int kHits = 8;
     int cnt = 0;

@@ -1736,9 +1736,10 @@ public:
         va.desc_frame = (long long)(W - 7) * (H - 7);
         va.nprop = kLearnedFrameProposals;
         // the register-blocked kernel takes the default form of the search (8 x 8 blocks, step 1, at
-        // most two centres); others, and windows beyond a warp's width, take the general kernel
+        // most two centres); others, windows beyond a warp's width, and thresholds that overflow fp32 (infinite
+        // distances are matches then, and mean "none" in that kernel) take the general kernel
         const bool fast_ps = para.B == 8 && para.psstep == 1 && para.psnum <= 2 && para.G <= 32 && !dwin &&
-                             va.ps_range <= kPsMaxRange;
+                             va.ps_range <= kPsMaxRange && std::isfinite(va.thSSE);
         size_t smem = 0;
         int warps = 4;
         for (; warps >= 1; warps /= 2) {

@@ -122,7 +122,7 @@ static cudaError_t launch_bm_est_t(const BMArgs &a, const EstLayout &L, int nfra
 
 int launch_bm_est(const BMArgs &a, int block_step, int last, int nframes, cudaStream_t s, cudaError_t *e)
 {
-    if (a.B != 8 || a.step != 1 || a.G < 2 || a.G > 32 || block_step > kEstMaxStep) return 0;
+    if (a.B != 8 || a.step != 1 || a.G < 2 || a.G > 32 || block_step > kEstMaxStep || !(a.thSSE <= kEstMaxThr)) return 0;
     // displacements per lane: 3 or 4, whichever leaves fewer slots of the team's 128 lanes unused
     const int span = 2 * a.range + 1;
     if (span * span >= 1 << 15) return 0;

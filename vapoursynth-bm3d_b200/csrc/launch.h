@@ -10,7 +10,7 @@ namespace bm3d {
 
 // Full search of 8 x 8 blocks (candidate step 1, 2 <= G <= 32, block step at most 8) with shared estimates and an
 // exact short list: launch_bm_full's lists.  last: position of a row's last reference block.  Returns 0
-// if the shape is not its own or its windows do not fit, else 1 and the status.
+// if the shape or the threshold is not its own or its windows do not fit, else 1 and the status.
 int launch_bm_est(const BMArgs &a, int block_step, int last, int nframes, cudaStream_t s, cudaError_t *e);
 cudaError_t launch_bm_full(const BMArgs &a, int nframes, size_t smem_bytes, cudaStream_t s);
 // Learned proposal (no reference counterpart): feature network forward into bf16 hidden /
@@ -31,7 +31,7 @@ cudaError_t launch_prop_sample(const float *frames, long long fstride, int ld, i
 cudaError_t launch_bm_learned(const BMArgs &a, const void *desc, int nprop, int nframes, size_t smem, cudaStream_t s);
 
 // fast: the register-blocked kernel (B = 8, ps_step 1, ps_num <= 2, G <= 32, no descriptors,
-// ps_range <= kPsMaxRange); same lists
+// ps_range <= kPsMaxRange, finite threshold); same lists
 cudaError_t launch_vbm_predict(const VBMArgs &a, bool fast, int nframes, size_t smem_bytes, cudaStream_t s);
 // Plain Final filter of BM3D frames (B = 8, G in {8, 16, 32}) with a run's image region in shared
 // memory; returns 0 if the shape is not its own or the region does not fit, else 1 and the status.
