@@ -8,7 +8,7 @@
 // into a second box in fixed point, which goes to the numerator plane once, with vector atomics.
 // Shared-memory atomics are native for 32-bit integers only (float and 64-bit ones are compare-and-swap
 // loops, 437 clocks a block and warp against 100), so a cell is two words of its own: a term is split
-// exactly into a multiple of 2^-13 and a multiple of 2^-32.
+// into a multiple of 2^-13 and the rest, rounded to a multiple of 2^-32 (terms from 2^-9 on lose nothing).
 //
 // Final (cf_box_kernel): a pair of warps per slot of 32 blocks (32 / G groups), both filtering the
 // reference and the source blocks at once as the halves of packed fp32 pairs (one instruction for
@@ -39,7 +39,8 @@ constexpr int kBoxRoundBits = 0x4b400000;
 // sum of a cell's words as a float
 __device__ __forceinline__ float box_value(int hi, int lo)
 {
-    // carry into the high word; both words are then exact in fp32 (the high one below 2^24 units)
+    // carry into the high word: the low one is then exact in fp32, the high one below 2^24 units, a sum of 2^11
+    // (a larger one is rounded twice)
     return __fmaf_rn(__int2float_rn(lo & 0x7ffff), kBoxLoUnit, __int2float_rn(hi + (lo >> 19)) * kBoxHiUnit);
 }
 
@@ -392,8 +393,9 @@ __device__ __forceinline__ float box_wiener_any(int at, float sg, int n, const C
     return box_wiener_direct(at, sg, n, dtab_for(a, n, false), dtab_for(a, n, true));
 }
 
-// the box, then the slot of block (0, 0), to the numerator plane
-__device__ __forceinline__ void box_flush(const int *acc, int cells, int slot0, int P, float *num, int ld, int y0, int x0, int bh, int bw)
+// the box, then the slot of block (0, 0), times `unit` (a power of two) to the numerator plane
+__device__ __forceinline__ void box_flush(const int *acc, int cells, int slot0, int P, float *num, int ld, int y0, int x0, int bh, int bw,
+                                          float unit)
 {
     const int qw = bw >> 2;
     for (int e = threadIdx.x; e < bh * qw; e += blockDim.x) {
@@ -401,12 +403,12 @@ __device__ __forceinline__ void box_flush(const int *acc, int cells, int slot0, 
         const int4 hi = *reinterpret_cast<const int4 *>(acc + yy * P + c), lo = *reinterpret_cast<const int4 *>(acc + cells + yy * P + c);
         float *d = num + (long long)(y0 + yy) * ld + x0 + c;
         if (hi.x | hi.y | hi.z | hi.w | lo.x | lo.y | lo.z | lo.w)
-            atomicAdd(reinterpret_cast<float4 *>(d), make_float4(box_value(hi.x, lo.x), box_value(hi.y, lo.y),
-                                                                 box_value(hi.z, lo.z), box_value(hi.w, lo.w)));
+            atomicAdd(reinterpret_cast<float4 *>(d), make_float4(box_value(hi.x, lo.x) * unit, box_value(hi.y, lo.y) * unit,
+                                                                 box_value(hi.z, lo.z) * unit, box_value(hi.w, lo.w) * unit));
     }
     if (threadIdx.x < 64) {
         const int e = slot0 + threadIdx.x;
-        if (acc[e] | acc[cells + e]) atomicAdd(num + (long long)(threadIdx.x >> 3) * ld + (threadIdx.x & 7), box_value(acc[e], acc[cells + e]));
+        if (acc[e] | acc[cells + e]) atomicAdd(num + (long long)(threadIdx.x >> 3) * ld + (threadIdx.x & 7), box_value(acc[e], acc[cells + e]) * unit);
     }
 }
 
@@ -557,7 +559,7 @@ __global__ void __launch_bounds__(NP * 64, 8 / NP) cf_box_kernel(CFArgs a, CFBox
     }
 
     __syncthreads();
-    box_flush(acc, cells, slot0, P, a.num[p] + f * a.frame_stride, a.ld, y0, x0, bh, bw);
+    box_flush(acc, cells, slot0, P, a.num[p] + f * a.frame_stride, a.ld, y0, x0, bh, bw, 1.0f);
 }
 
 // ---- Basic: hard threshold ------------------------------------------------------------------------------
@@ -566,6 +568,49 @@ __global__ void __launch_bounds__(NP * 64, 8 / NP) cf_box_kernel(CFArgs a, CFBox
 // Bound: the shared-memory pipe (random-row loads of the blocks, transposes, and four native atomics a
 // pixel pair: 6.7 k of a step's 25 k clocks are atomics).  1920x1080 RGB x 8, step 4, G = 16: 12.6 ms with
 // per-lane gathers and float atomics on the plane (cf_fast_kernel), 8.3 ms now.
+
+// A term is a pixel over its group's kept count, so its size follows the clip's, and an absolute grid would keep
+// fewer bits of a clip of small values than fp32 sums do.  So
+// - a tile whose largest staged magnitude is below kTileMin is filtered in units that put it in [32, 64), a power
+//   of two: its terms are those of the clip, scaled;
+// - a group whose terms are still below kBoxMin (a dark part of a bright tile) goes to the plane directly, as
+//   blocks of large terms do.
+// The grid's rounding is then at most 2^-19 of the largest term of a group's first block, and usually far less: the
+// test takes one coefficient's share of it.  A pixel averages the roundings of dozens of terms.
+constexpr float kTileMin = 0.0625f;                                            // 2^-4
+constexpr float kBoxMin = 6.103515625e-5f;                                     // 2^-14
+
+__device__ __forceinline__ unsigned abs_bits(float v) { return __float_as_uint(v) & 0x7fffffffu; }
+
+// bits of a tile's scale, from the bits of its largest magnitude; limited so that neither the scale nor its inverse
+// underflows
+__device__ __forceinline__ unsigned box_scale_bits(unsigned top)
+{
+    return top < __float_as_uint(kTileMin) ? (unsigned)min(259 - (int)(top >> 23), 253) << 23 : 127u << 23;
+}
+
+// the block of slot A (low halves) and of slot B at a place, one of which may not go to the box: each to the cells
+// (at ca, cb, and 4 further on for the second pixel) or to the plane (at na, nb) times `down`
+__device__ __noinline__ void box_add_apart(f2 e0, f2 e1, int *ca, int *cb, int low, float *na, float *nb, float down, bool apartA, bool apartB)
+{
+    float a0, b0, a1, b1;
+    upk(e0, a0, b0);
+    upk(e1, a1, b1);
+    const bool fa = !apartA && __all_sync(0xffffffffu, fabsf(a0) < kBoxMax && fabsf(a1) < kBoxMax);
+    const bool fb = !apartB && __all_sync(0xffffffffu, fabsf(b0) < kBoxMax && fabsf(b1) < kBoxMax);
+    if (fa || fb) {
+        box_add(pk(fa ? a0 : 0.0f, fb ? b0 : 0.0f), ca, cb, low);
+        box_add(pk(fa ? a1 : 0.0f, fb ? b1 : 0.0f), ca + 4, cb + 4, low);
+    }
+    if (!fa) {
+        atomicAdd(na, a0 * down);
+        atomicAdd(na + 4, a1 * down);
+    }
+    if (!fb) {
+        atomicAdd(nb, b0 * down);
+        atomicAdd(nb + 4, b1 * down);
+    }
+}
 
 // hard threshold of both halves of x, counted in the halves of kept
 __device__ __forceinline__ f2 keep2(f2 x, float ta, float tb, int &kept)
@@ -727,7 +772,9 @@ __global__ void __launch_bounds__(NP * 64, 8 / NP) cf_boxh_kernel(CFArgs a, CFBo
     f2 *tr = reinterpret_cast<f2 *>(smem);
     int *acc = reinterpret_cast<int *>(tr + NP * kT);                  // high words, then low words
     float *box = reinterpret_cast<float *>(acc + 2 * cells);
-    int *red = reinterpret_cast<int *>(box + cells) + pair * 2 * GPW;  // [group of the slots][warp]
+    unsigned *tops = reinterpret_cast<unsigned *>(box + cells);        // [warp]
+    int *red = reinterpret_cast<int *>(tops + 2 * NP) + pair * 6 * GPW;  // [group of the slots][warp]: kept counts,
+    int *redA = red + 2 * GPW, *redB = redA + 2 * GPW;                 // magnitude bits of the first blocks of A and of B
     const float *src = a.src[p] + f * a.frame_stride;
     const int h = lane & 1;
     const int blk = 16 * role + (lane >> 1);        // the lane's block of a slot: group sub, place z
@@ -760,7 +807,21 @@ __global__ void __launch_bounds__(NP * 64, 8 / NP) cf_boxh_kernel(CFArgs a, CFBo
     }
     for (int e = threadIdx.x; e < (cells >> 1); e += NP * 64) reinterpret_cast<int4 *>(acc)[e] = make_int4(0, 0, 0, 0);
     tc::cp_async_wait_all();
+    // largest finite magnitude of the plane's pixels among the thread's own copies, then of the tile
+    unsigned top = 0u;
+    for (int e = threadIdx.x; e < chunks; e += NP * 64) {
+        const int yy = e / qw, c = 4 * (e - yy * qw), m = e - (chunks - 16);
+        const float4 v = *reinterpret_cast<const float4 *>(box + (m < 0 ? yy * P + c : slot0 + 4 * m));
+        const unsigned u[4] = {abs_bits(v.x), abs_bits(v.y), abs_bits(v.z), abs_bits(v.w)};
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+            if (u[k] < 0x7f800000u && (m >= 0 || x0 + c + k < a.W)) top = max(top, u[k]);
+    }
+    top = __reduce_max_sync(0xffffffffu, top);
+    if (lane == 0) tops[warp] = top;
     __syncthreads();
+    const unsigned sb = box_scale_bits(__reduce_max_sync(0xffffffffu, tops[lane & (2 * NP - 1)]));
+    const float up = __uint_as_float(sb), down = __uint_as_float((254u << 23) - sb);
 
     f2 *tb = tr + pair * kT + blk * kBT;
     const int sy = lane & 7, sx = lane >> 3;        // the lane's pixel of a block in the scatter (and column sx + 4)
@@ -791,7 +852,14 @@ __global__ void __launch_bounds__(NP * 64, 8 / NP) cf_boxh_kernel(CFArgs a, CFBo
             const int ma = q < gA ? min(a.count[grpA + q], G) : 0, mb = q < gB ? min(a.count[grpB + q], G) : 0;
             const int at = pair * kT + q * G * kBT + col;
             const int kept = box_hard_pair<G>(at, a, p, fxy, ma, mb);
-            if (lane == 0) red[2 * q + role] = kept;
+            float ca, cb;
+            upk(reinterpret_cast<f2 *>(smem)[at], ca, cb);
+            const unsigned ta = __reduce_max_sync(0xffffffffu, abs_bits(ca)), tb0 = __reduce_max_sync(0xffffffffu, abs_bits(cb));
+            if (lane == 0) {
+                red[2 * q + role] = kept;
+                redA[2 * q + role] = (int)ta;
+                redB[2 * q + role] = (int)tb0;
+            }
         }
         pair_barrier(1 + pair);
         const int kept = red[2 * sub] + red[2 * sub + 1], kA = kept & 0xffff, kB = kept >> 16;
@@ -800,16 +868,24 @@ __global__ void __launch_bounds__(NP * 64, 8 / NP) cf_boxh_kernel(CFArgs a, CFBo
             if (sub < gB) a.retained[(long long)p * a.ngroups + grpB + sub] = kB;
         }
         const float dA = kA < 1 ? 1.0f : __fdiv_rn(1.0f, (float)kA), dB = kB < 1 ? 1.0f : __fdiv_rn(1.0f, (float)kB);
-        box_inverse2(tb, pk(actA ? __fdiv_rn(dA, a.amp[na - 1]) : 0.0f, actB ? __fdiv_rn(dB, a.amp[nb - 1]) : 0.0f), actA, actB, h);
+        const float wA = actA ? __fdiv_rn(dA, a.amp[na - 1]) * up : 0.0f, wB = actB ? __fdiv_rn(dB, a.amp[nb - 1]) * up : 0.0f;
+        // a pixel is, on the mean square, at least as large as any one of the block's coefficients
+        const float tA = __int_as_float(max(redA[2 * sub], redA[2 * sub + 1])) * wA;
+        const float tB = __int_as_float(max(redB[2 * sub], redB[2 * sub + 1])) * wB;
+        const bool apartA = actA && tA > 0.0f && tA < kBoxMin, apartB = actB && tB > 0.0f && tB < kBoxMin;
+        const unsigned apart = __ballot_sync(0xffffffffu, apartA || apartB), places = __ballot_sync(0xffffffffu, actA || actB);
+        box_inverse2(tb, pk(wA, wB), actA, actB, h);
         __syncwarp();
         // aggregation, four blocks (two places of both slots) per step
         const f2 *v = tr + pair * kT + 16 * role * kBT + lane;
         int *cell = acc + sy * P + sx, *cell0 = acc + sy * 8 + sx;
+        unsigned later = 0u;
 #pragma unroll
         for (int i = 0; i < 16; i += 2) {
             f2 e[4];
             int oa[2], ob[2];
             bool fits = true;
+            if (!(places >> 2 * i & 15u)) continue;     // past the groups' ends
 #pragma unroll
             for (int k = 0; k < 2; ++k) {
                 oa[k] = __shfl_sync(0xffffffffu, offA, 2 * (i + k));
@@ -823,7 +899,7 @@ __global__ void __launch_bounds__(NP * 64, 8 / NP) cf_boxh_kernel(CFArgs a, CFBo
                 upk(e[k], u, w);
                 fits = fits && fabsf(u) < kBoxMax && fabsf(w) < kBoxMax;
             }
-            if (__all_sync(0xffffffffu, fits)) {
+            if (!apart && __all_sync(0xffffffffu, fits)) {
 #pragma unroll
                 for (int k = 0; k < 2; ++k) {
                     int *ca = (oa[k] < slot0 ? cell : cell0) + oa[k], *cb = (ob[k] < slot0 ? cell : cell0) + ob[k];
@@ -831,21 +907,18 @@ __global__ void __launch_bounds__(NP * 64, 8 / NP) cf_boxh_kernel(CFArgs a, CFBo
                     box_add(e[2 * k + 1], ca + 4, cb + 4, cells);
                 }
             } else {
-#pragma unroll 1
-                for (int k = 0; k < 2; ++k) {
-                    const uint32_t qa = __shfl_sync(0xffffffffu, posA, 2 * (i + k)), qb = __shfl_sync(0xffffffffu, posB, 2 * (i + k));
-                    float *num = a.num[p] + f * a.frame_stride;
-                    float *na_ = num + (long long)(unpack_y(qa) + sy) * a.ld + unpack_x(qa) + sx;
-                    float *nb_ = num + (long long)(unpack_y(qb) + sy) * a.ld + unpack_x(qb) + sx;
-                    float u, w;
-                    upk(v[(i + k) * kBT], u, w);
-                    atomicAdd(na_, u);
-                    atomicAdd(nb_, w);
-                    upk(v[(i + k) * kBT + 32], u, w);
-                    atomicAdd(na_ + 4, u);
-                    atomicAdd(nb_ + 4, w);
-                }
+                later |= 3u << i;
             }
+        }
+        // places with a block that the box does not take: each block to its own destination
+        for (; later; later &= later - 1) {
+            const int i = __ffs(later) - 1;
+            const int ia = __shfl_sync(0xffffffffu, offA, 2 * i), ib = __shfl_sync(0xffffffffu, offB, 2 * i);
+            const uint32_t qa = __shfl_sync(0xffffffffu, posA, 2 * i), qb = __shfl_sync(0xffffffffu, posB, 2 * i);
+            float *num = a.num[p] + f * a.frame_stride + (long long)sy * a.ld + sx;
+            box_add_apart(v[i * kBT], v[i * kBT + 32], (ia < slot0 ? cell : cell0) + ia, (ib < slot0 ? cell : cell0) + ib, cells,
+                          num + (long long)unpack_y(qa) * a.ld + unpack_x(qa), num + (long long)unpack_y(qb) * a.ld + unpack_x(qb), down,
+                          __shfl_sync(0xffffffffu, apartA, 2 * i), __shfl_sync(0xffffffffu, apartB, 2 * i));
         }
         if (h == 0) {
             float *wm = a.wmap[p] + f * a.frame_stride;
@@ -856,7 +929,7 @@ __global__ void __launch_bounds__(NP * 64, 8 / NP) cf_boxh_kernel(CFArgs a, CFBo
     }
 
     __syncthreads();
-    box_flush(acc, cells, slot0, P, a.num[p] + f * a.frame_stride, a.ld, y0, x0, bh, bw);
+    box_flush(acc, cells, slot0, P, a.num[p] + f * a.frame_stride, a.ld, y0, x0, bh, bw, down);
 }
 
 // ---- V-BM3D: the same warp pairs without a box -----------------------------------------------------------

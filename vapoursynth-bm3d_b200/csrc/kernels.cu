@@ -191,7 +191,7 @@ static int cf_box_fit(const CFArgs &a, CFBox &g, int step, int G, int NP, int re
             const int w = (2 * g.range + 8 + (nx - 1) * step + 3 + 3) & ~3;
             const int rows = std::min(a.H, 2 * g.range + 8 + (ny - 1) * step);
             const int pitch = w + ((12 - (w & 7)) & 7);      // 4 mod 8: a scatter step's eight rows in distinct banks
-            const size_t bytes = (size_t)NP * 32 * kBT * 8 + ((size_t)rows * pitch + 64) * cell + (size_t)NP * 2 * gpw * 4;
+            const size_t bytes = (size_t)NP * 32 * kBT * 8 + ((size_t)rows * pitch + 64) * cell + (size_t)NP * 2 * gpw * 4 * (a.wiener ? 1 : 3) + (a.wiener ? 0 : (size_t)NP * 2 * 4);
             if (bytes > cap) break;
             const int steps = (ny * (nx / gpw) + per_step - 1) / per_step;
             const int tx = (g.nbx + nx - 1) / nx, ty = (g.nby + ny - 1) / ny;
