@@ -932,9 +932,10 @@ __global__ void __launch_bounds__(NP * 64, 8 / NP) cf_boxh_kernel(CFArgs a, CFBo
     box_flush(acc, cells, slot0, P, a.num[p] + f * a.frame_stride, a.ld, y0, x0, bh, bw, down);
 }
 
-// ---- V-BM3D: the same warp pairs without a box -----------------------------------------------------------
-// A group's blocks lie in up to 2 radius + 1 frames, so there is no box to stage: blocks are read from and added to
-// the planes one per warp step (lane = row and column of half a block), through the transpose buffer.
+// ---- the same warp pairs without a box --------------------------------------------------------------------
+// V-BM3D, whose groups' blocks lie in up to 2 radius + 1 frames, and search windows whose box holds too few groups:
+// blocks are read from and added to the planes one per warp step (lane = row and column of half a block), through
+// the transpose buffer.
 // Bound: latency of the steps and the L2's atomics.  1280x720 YUV x 7, radius 3, Final, G = 8: 7.4 ms
 // with per-lane gathers and atomics (cf_fast_kernel), 4.8 ms here.
 

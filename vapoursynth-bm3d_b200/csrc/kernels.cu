@@ -176,26 +176,42 @@ cudaError_t launch_vbm_predict(const VBMArgs &a, bool fast, int nframes, size_t 
 
 int cf_fast_supported(int B, int G) { return B == 8 && (G == 8 || G == 16 || G == 32); }
 
-// Tile of reference blocks for cf_box_kernel / cf_boxh_kernel with NP warp pairs and at most `cap` bytes of shared memory
-// per CTA (0: none fits); fills the geometry.  A pair takes one slot of 32 / G groups per step (Basic: two), and staging
-// and flushing the box cost about half a step: the tile with the least waves x (steps + 1/2) is taken, where
-// `resident` CTAs run at once (so that a small frame gets small tiles and all SMs; 352x288 at profile fast,
-// 1,584 groups: 34 us with the largest tile, 30 us).
-static int cf_box_fit(const CFArgs &a, CFBox &g, int step, int G, int NP, int resident, size_t cap, size_t *smem)
+// Two CTAs of four warp pairs per SM: shared memory of one, and how many run at once
+constexpr int kBoxPairs = 4, kBoxCap = 115712, kBoxResident = 2 * 148;
+
+// Tile of reference blocks for cf_box_kernel / cf_boxh_kernel; fills the geometry and returns whether the box form is the
+// one to take.  A pair takes one slot of 32 / G groups per step (Basic: two), and staging and flushing the box cost about
+// half a step: the tile with the least waves x (steps + 1/2) is taken (so that a small frame gets small tiles and
+// all SMs; 352x288 at profile fast, 1,584 groups: 34 us with the largest tile, 30 us).
+// launch_cf_pair takes the others:
+// - Where no tile that fits fills three quarters of a step, pairs idle and a box is staged for a few groups.
+//   1920x1080 YUV x 3, box and pairs: Basic, range 24, step 4, G = 16 (one slot of eight) 20.2 and 3.5 ms; range 20 (six
+//   of eight) 4.9 and 3.5 ms, still ahead of a warp per group (5.4 ms); Final, range 20, step 4, G = 16 (one of four) 15.1
+//   and 5.2 ms.  (Three CTAs of two pairs, or one of four in all shared memory, gain nothing on the pairs at any range:
+//   Final, range 36, step 8, G = 8: 2.47 and 0.70 ms.)
+// - Where a window has fewer than 4 G candidates, most lists are short and of any length, and the slow direct
+//   sums of one pair hold up its CTA's tile.  640x480, step 3: Basic, G = 16, range 3 184 and 141 us, range 4 143 and
+//   137 us; Final, G = 32, range 5 794 and 489 us, range 6 485 and 515 us.
+static bool cf_box_fit(const CFArgs &a, CFBox &g, int step, int G, size_t *smem)
 {
     const int gpw = 32 / G;
-    const int cell = a.wiener ? 16 : 12, per_step = a.wiener ? NP : 2 * NP;   // bytes of a cell, slots of a step
+    const int cell = a.wiener ? 16 : 12, per_step = a.wiener ? kBoxPairs : 2 * kBoxPairs;   // bytes of a cell, slots of a step
+    const int span = 2 * g.range + 1;
+    if (span * span < 4 * G) return false;
     double best = 0.0;
+    int most = 0;                                            // slots of the largest tile
     for (int ny = 1; ny <= 8; ++ny)
         for (int nx = gpw; nx * ny <= 128; nx += gpw) {
             const int w = (2 * g.range + 8 + (nx - 1) * step + 3 + 3) & ~3;
             const int rows = std::min(a.H, 2 * g.range + 8 + (ny - 1) * step);
             const int pitch = w + ((12 - (w & 7)) & 7);      // 4 mod 8: a scatter step's eight rows in distinct banks
-            const size_t bytes = (size_t)NP * 32 * kBT * 8 + ((size_t)rows * pitch + 64) * cell + (size_t)NP * 2 * gpw * 4 * (a.wiener ? 1 : 3) + (a.wiener ? 0 : (size_t)NP * 2 * 4);
-            if (bytes > cap) break;
-            const int steps = (ny * (nx / gpw) + per_step - 1) / per_step;
+            const size_t bytes = (size_t)kBoxPairs * 32 * kBT * 8 + ((size_t)rows * pitch + 64) * cell +
+                                 (size_t)kBoxPairs * 2 * gpw * 4 * (a.wiener ? 1 : 3) + (a.wiener ? 0 : (size_t)kBoxPairs * 2 * 4);
+            if (bytes > kBoxCap) break;
+            const int slots = ny * (nx / gpw), steps = (slots + per_step - 1) / per_step;
+            most = std::max(most, slots);
             const int tx = (g.nbx + nx - 1) / nx, ty = (g.nby + ny - 1) / ny;
-            double waves = (double)tx * ty * g.nplanes * (double)(a.ngroups / a.blocks_per_frame) / resident;
+            double waves = (double)tx * ty * g.nplanes * (double)(a.ngroups / a.blocks_per_frame) / kBoxResident;
             if (waves < 6.0) waves = std::ceil(waves);
             const double cost = waves * (steps + 0.5);
             if (best > 0.0 && cost >= best) continue;
@@ -206,40 +222,30 @@ static int cf_box_fit(const CFArgs &a, CFBox &g, int step, int G, int NP, int re
             g.pitch = pitch;
             *smem = bytes;
         }
-    return best > 0.0;
-}
-
-template <int G, int NP>
-static cudaError_t launch_cf_box_t(const CFArgs &a, const CFBox &g, size_t smem, cudaStream_t s)
-{
-    auto kernel = a.wiener ? cf_box_kernel<G, NP> : cf_boxh_kernel<G, NP>;
-    cudaError_t e;
-    if ((e = allow_smem(kernel, smem)) != cudaSuccess) return e;
-    const long long frames = a.ngroups / a.blocks_per_frame;
-    COUNT_LAUNCH();
-    kernel<<<dim3((unsigned)(frames * g.tx * g.ty), g.nplanes), NP * 64, smem, s>>>(a, g);
-    return cudaGetLastError();
+    return 4 * most >= 3 * per_step;
 }
 
 template <int G>
-static int launch_cf_box_g(const CFArgs &a, CFBox g, int step, cudaStream_t s, cudaError_t *e)
+static int launch_cf_box_t(const CFArgs &a, CFBox g, int step, cudaStream_t s, cudaError_t *e)
 {
     size_t smem = 0;
-    constexpr int sms = 148;
-    // two CTAs of four pairs per SM; else three of two pairs; else one CTA of four pairs
-    if (cf_box_fit(a, g, step, G, 4, 2 * sms, 115712, &smem)) return *e = launch_cf_box_t<G, 4>(a, g, smem, s), 1;
-    if (cf_box_fit(a, g, step, G, 2, 3 * sms, 76800, &smem)) return *e = launch_cf_box_t<G, 2>(a, g, smem, s), 1;
-    if (cf_box_fit(a, g, step, G, 4, sms, 232448, &smem)) return *e = launch_cf_box_t<G, 4>(a, g, smem, s), 1;
-    return 0;
+    if (!cf_box_fit(a, g, step, G, &smem)) return 0;
+    auto kernel = a.wiener ? cf_box_kernel<G, kBoxPairs> : cf_boxh_kernel<G, kBoxPairs>;
+    if ((*e = allow_smem(kernel, smem)) != cudaSuccess) return 1;
+    const long long frames = a.ngroups / a.blocks_per_frame;
+    COUNT_LAUNCH();
+    kernel<<<dim3((unsigned)(frames * g.tx * g.ty), g.nplanes), kBoxPairs * 64, smem, s>>>(a, g);
+    *e = cudaGetLastError();
+    return 1;
 }
 
 int launch_cf_box(const CFArgs &a, const CFBox &g, int step, cudaStream_t s, cudaError_t *e)
 {
     if (a.B != 8 || a.vbm3d) return 0;
     switch (a.G) {
-    case 8: return launch_cf_box_g<8>(a, g, step, s, e);
-    case 16: return launch_cf_box_g<16>(a, g, step, s, e);
-    case 32: return launch_cf_box_g<32>(a, g, step, s, e);
+    case 8: return launch_cf_box_t<8>(a, g, step, s, e);
+    case 16: return launch_cf_box_t<16>(a, g, step, s, e);
+    case 32: return launch_cf_box_t<32>(a, g, step, s, e);
     default: return 0;
     }
 }

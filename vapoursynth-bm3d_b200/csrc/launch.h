@@ -33,10 +33,10 @@ cudaError_t launch_bm_learned(const BMArgs &a, const void *desc, int nprop, int 
 // fast: the register-blocked kernel (B = 8, ps_step 1, ps_num <= 2, G <= 32, no descriptors,
 // ps_range <= kPsMaxRange, finite threshold); same lists
 cudaError_t launch_vbm_predict(const VBMArgs &a, bool fast, int nframes, size_t smem_bytes, cudaStream_t s);
-// Plain Final filter of BM3D frames (B = 8, G in {8, 16, 32}) with a run's image region in shared
-// memory; returns 0 if the shape is not its own or the region does not fit, else 1 and the status.
+// Plain Basic and Final filters of BM3D frames (B = 8, G in {8, 16, 32}) with a tile's image region in shared
+// memory; returns 0 if the shape is not its own or launch_cf_pair is the faster form, else 1 and the status.
 int launch_cf_box(const CFArgs &a, const CFBox &g, int step, cudaStream_t s, cudaError_t *e);
-// The same warp pairs without a staged region: V-BM3D groups, and regions too large to stage (B = 8, G in
+// The same warp pairs without a staged region: V-BM3D groups, wide and very small search windows (B = 8, G in
 // {8, 16, 32}).
 cudaError_t launch_cf_pair(const CFArgs &a, cudaStream_t s);
 // Fast collaborative filter (B = 8, G in {8, 16, 32}, any group length n <= G); sizes its own
