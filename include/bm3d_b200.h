@@ -209,6 +209,9 @@ BM3D_API int bm3d_debug_retained_counts(bm3d_filter *filter, int k, int *counts,
  * register path of the 8x8 / n in {8,16,32} kernels.  inverse = 0 forward (REDFT10 definition),
  * 1 inverse (REDFT01). */
 BM3D_API int bm3d_debug_dct3d(float *groups, int ngroups, int n, int block_size, int inverse, int fast);
+/* Wiener weights r2 / (r2 + sigma2) of n pairs (all arrays in HOST memory): weights as the plain Final filters form
+ * them, quotients by IEEE division. */
+BM3D_API int bm3d_debug_wiener_weights(const float *r2, const float *sigma2, int n, float *weights, float *quotients);
 
 /* ---- Learned block-matching proposal (precision = "learned"); no reference counterpart --------
  * Network: 3x3 conv 1 -> 16 channels, ReLU, 3x3 conv 16 -> 16, bf16 activations; descriptor of

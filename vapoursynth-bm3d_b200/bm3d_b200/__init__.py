@@ -354,6 +354,17 @@ class _Core:
 core = _Core()
 
 
+def wiener_weights(r2, sigma2):
+    """Wiener weights r2 / (r2 + sigma2) of float32 arrays: as the plain Final filters form them, and by division."""
+    a, b = np.ascontiguousarray(r2, np.float32), np.ascontiguousarray(sigma2, np.float32)
+    w, q = np.empty_like(a), np.empty_like(a)
+    rc = capi.lib().bm3d_debug_wiener_weights(*(v.ctypes.data_as(C.POINTER(C.c_float)) for v in (a, b)), a.size,
+                                              *(v.ctypes.data_as(C.POINTER(C.c_float)) for v in (w, q)))
+    if rc != 0:
+        raise Error(capi.last_error())
+    return w, q
+
+
 def dct3d(groups, inverse=False, fast=False):
     """Runs the library's 3-D transform on groups [g][n][B][B] (float32, host); returns a copy."""
     g = np.ascontiguousarray(groups, dtype=np.float32).copy()

@@ -20,7 +20,7 @@ EXPORTS = [
     "bm3d_debug_reference_fp64", "bm3d_debug_bm_tc_counts", "bm3d_proposal_default_weights",
     "bm3d_proposal_descriptors", "bm3d_proposal_gradients", "bm3d_proposal_train", "bm3d_proposal_match",
     "bm3d_debug_proposal_sets", "bm3d_debug_threshold_rechecks", "bm3d_debug_set_recheck_band",
-    "bm3d_debug_retained_counts",
+    "bm3d_debug_retained_counts", "bm3d_debug_wiener_weights",
 ]
 
 
@@ -90,6 +90,7 @@ def lib():
     L.bm3d_debug_launch_count.restype = C.c_int64
     L.bm3d_debug_reference_fp64.argtypes = [C.c_void_p, C.c_int, P(C.c_double), C.c_int64]
     L.bm3d_debug_dct3d.argtypes = [P(C.c_float), C.c_int, C.c_int, C.c_int, C.c_int, C.c_int]
+    L.bm3d_debug_wiener_weights.argtypes = [P(C.c_float), P(C.c_float), C.c_int, P(C.c_float), P(C.c_float)]
     L.bm3d_basic_noalloc.argtypes = [C.c_void_p, C.c_void_p, C.c_int, C.c_int, C.c_int64, C.c_char_p, C.c_double,
                                      C.c_void_p]
     _lib = L

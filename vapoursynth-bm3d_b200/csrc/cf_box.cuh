@@ -163,11 +163,17 @@ __device__ __forceinline__ void idct_sets(const float (&X)[N], F &&f)
     }
 }
 
-// Wiener weights w[i] = r2[i] / (r2[i] + sg): reciprocal estimate, quotient, and one correction by the exact
+// Wiener weights w[i] = r2[i] / (r2[i] + sg): reciprocal estimate, quotient, and one correction by the
 // remainder (Markstein, IBM J. Res. Dev. 34, 1990), which rounds as the division does but for quotients
-// within a few 2^-46 of a tie.  EXACT: the division itself, a dozen instructions and a branch each.  The estimate
-// underflows for divisors from 2^126 on: `top` collects the largest, and a column that has one is redone.
+// within 2^-45 of a tie (of 4 M random pairs, none to a few, by one unit), as long as the remainder is exact: for
+// r2 from 2^-102 on.  Below, the quotient stays within three units.
+// EXACT: the division itself, a dozen instructions and a branch each.  A column takes it
+// - where a divisor reaches 2^126 and its estimate underflows: `top` collects the largest, and the column is redone;
+// - where sg is below kWienerLow, so that an r2 below 2^-102 may have a weight that counts (else it is below 2^-42):
+//   `top` starts at wiener_top(sg), the limit.
 constexpr float kWienerTop = 4.2535296e37f;       // 2^125
+constexpr float kWienerLow = 8.6736174e-19f;      // 2^-60
+__device__ __forceinline__ float wiener_top(float sg) { return sg < kWienerLow ? kWienerTop : 0.0f; }
 
 template <bool EXACT, int C>
 __device__ __forceinline__ void wiener_weights(const float (&r2)[C], float sg, float (&w)[C], float &top)
@@ -357,7 +363,7 @@ __device__ __noinline__ float box_wiener(int at, float sg)
 {
     extern __shared__ __align__(16) float smem[];
     f2 *t = reinterpret_cast<f2 *>(smem) + at;
-    float top = 0.0f;
+    float top = wiener_top(sg);
     const float l2 = wiener_column<N, false>(t, kBT, sg, top);
     return top < kWienerTop ? l2 : wiener_column_exact<N>(t, kBT, sg);
 }

@@ -82,7 +82,7 @@ __device__ __forceinline__ void mid_transform(T *v, int stride, int B, const flo
 template <int N>
 __device__ __forceinline__ float mid_z(f2 *v, int stride, float sg, float)
 {
-    float top = 0.0f;
+    float top = wiener_top(sg);
     const float l2 = wiener_column<N, false>(v, stride, sg, top);
     return top < kWienerTop ? l2 : wiener_column_exact<N>(v, stride, sg);
 }

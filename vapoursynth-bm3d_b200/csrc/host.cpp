@@ -2557,4 +2557,21 @@ BM3D_API int bm3d_debug_dct3d(float *groups, int ngroups, int n, int B, int inve
     });
 }
 
+BM3D_API int bm3d_debug_wiener_weights(const float *r2, const float *sigma2, int n, float *weights, float *quotients)
+{
+    g_error.clear();
+    if (!r2 || !sigma2 || !weights || !quotients || n < 1) return fail(BM3D_ERR_STATE, "bad arguments");
+    return guarded([&]() -> int {
+        DevBuf buf;
+        float *d = static_cast<float *>(buf.get(sizeof(float) * 4 * (size_t)n));
+        CU(cudaMemcpy(d, r2, sizeof(float) * n, cudaMemcpyHostToDevice));
+        CU(cudaMemcpy(d + n, sigma2, sizeof(float) * n, cudaMemcpyHostToDevice));
+        CU(launch_wiener_test(d, d + n, n, d + 2 * (size_t)n, d + 3 * (size_t)n, 0));
+        CU(cudaDeviceSynchronize());
+        CU(cudaMemcpy(weights, d + 2 * (size_t)n, sizeof(float) * n, cudaMemcpyDeviceToHost));
+        CU(cudaMemcpy(quotients, d + 3 * (size_t)n, sizeof(float) * n, cudaMemcpyDeviceToHost));
+        return (int)BM3D_OK;
+    });
+}
+
 }  // extern "C"

@@ -649,4 +649,23 @@ cudaError_t launch_dct3d_test(float *data, int ngroups, int n, int B, int invers
     return cudaGetLastError();
 }
 
+// each pair as a column of one coefficient
+__global__ void wiener_test_kernel(const float *r2, const float *sg, int n, float *w, float *exact)
+{
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const float r[1] = {r2[i]};
+    float v[1], q[1], top = wiener_top(sg[i]), unused = 0.0f;
+    wiener_weights<false, 1>(r, sg[i], v, top);
+    wiener_weights<true, 1>(r, sg[i], q, unused);
+    w[i] = top < kWienerTop ? v[0] : q[0];
+    exact[i] = q[0];
+}
+
+cudaError_t launch_wiener_test(const float *r2, const float *sg, int n, float *w, float *exact, cudaStream_t s)
+{
+    wiener_test_kernel<<<(n + 255) / 256, 256, 0, s>>>(r2, sg, n, w, exact);
+    return cudaGetLastError();
+}
+
 }  // namespace bm3d

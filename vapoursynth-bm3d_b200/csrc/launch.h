@@ -60,6 +60,8 @@ cudaError_t launch_vstack(const VStackArgs &a, int nframes, cudaStream_t s);
 cudaError_t launch_dct3d_test(float *data, int ngroups, int n, int B, int inverse, int fast,
                               const float *odd_all, const float *dtab, const int *dtab_off,
                               cudaStream_t s);
+// Wiener weights of n (squared coefficient, variance) pairs as the filters form them, and by division.
+cudaError_t launch_wiener_test(const float *r2, const float *sg, int n, float *w, float *exact, cudaStream_t s);
 
 int cf_fast_supported(int B, int G);
 
