@@ -152,11 +152,11 @@ BM3D_API void bm3d_set_log_callback(bm3d_log_fn fn, void *user);
  * loads the library's device code until the process exits.  A plane that needs more (1920x1080
  * fits at every profile; a 3840x2160 plane does not) is rejected with BM3D_ERR_UNSUPPORTED and a
  * message that gives the size it needed.  The first call on a device sets that device up (finds the
- * array's device address and copies constant tables with synchronous copies): make that first call
- * before any stream capture on the device.  All calls share the one array, which keeps the last
- * call's contents; each call clears what must start at zero, but calls that overlap on the GPU
- * (different streams, or host threads that do not order their calls) race and corrupt each
- * other's results, so order them on one stream.  The set-up is not redone after a device reset:
+ * array's device address, copies constant tables with synchronous copies, creates an event): make that first call
+ * before any stream capture on the device.  All calls share the one array: calls on one
+ * device run one after the other on the GPU, whatever streams and host threads they come from (each
+ * stream waits for the call before).  A call captured into a graph is outside that order: do not let
+ * its replays overlap other calls or each other.  The set-up is not redone after a device reset:
  * do not call cudaDeviceReset on a device after the first call on it. */
 BM3D_API int bm3d_basic_noalloc(const float *src, float *dst, int width, int height, int64_t stride,
                                 const char *profile, double sigma, void *cuda_stream);

@@ -13,10 +13,12 @@
 // The array has a fixed size, kScratchBytes (48 MiB: a 1920x1080 plane at every profile fits),
 // and every GPU that loads the library's device code holds it until the process exits.  All calls
 // share it and it keeps the contents of the last call, so each call clears the accumulators that
-// must start at zero, and two calls that overlap on the GPU (different streams, or threads that
-// do not order their calls) race with each other.  The set-up of a device (the array's address
-// and the constant tables) is done once per process: a caller that resets the device
-// (cudaDeviceReset) after its first call gets a reloaded, zeroed array and must not call again.
+// must start at zero.  Calls of one device run one after the other on the GPU, whatever streams and
+// threads they come from: each waits, on its stream, for an event recorded behind the one before.
+// (A call captured into a graph can neither wait for an event outside nor be waited for: its replays
+// are the caller's to order.)  The set-up of a device (the array's address, the constant tables and
+// the event) is done once per process: a caller that resets the device (cudaDeviceReset) after its
+// first call gets a reloaded, zeroed array and must not call again.
 
 #include "bm3d_b200.h"
 
@@ -62,6 +64,8 @@ long long round64(long long n) { return (n + 63) / 64 * 64; }
 
 std::mutex g_setup_mutex;
 float *g_dev_scratch[kMaxDevices];       // device address of the array, per device (set-up done)
+std::mutex g_call_mutex[kMaxDevices];    // held while a call of the device is enqueued
+cudaEvent_t g_last_call[kMaxDevices];    // recorded behind the device's last call
 
 // Host image of the table region, built once.
 float g_table_image[kTableFloats];
@@ -107,10 +111,40 @@ int setup_device(int dev, float **out)
     if (e != cudaSuccess) return set_error(BM3D_ERR_CUDA, cuda_text("cudaGetSymbolAddress", e));
     if ((e = cudaMemcpy(ptr, g_table_image, sizeof(g_table_image), cudaMemcpyHostToDevice)) != cudaSuccess)
         return set_error(BM3D_ERR_CUDA, cuda_text("table upload", e));
+    if ((e = cudaEventCreateWithFlags(&g_last_call[dev], cudaEventDisableTiming)) != cudaSuccess)
+        return set_error(BM3D_ERR_CUDA, cuda_text("cudaEventCreateWithFlags", e));
     g_dev_scratch[dev] = ptr;
     *out = ptr;
     return BM3D_OK;
 }
+
+// A call's turn on the array: the stream waits for the call before, and what was enqueued by the end of
+// the scope is what the next call waits for.
+class Turn {
+public:
+    Turn(int dev, cudaStream_t s) : lock_(g_call_mutex[dev]), event_(g_last_call[dev]), stream_(s) {}
+    cudaError_t begin()
+    {
+        cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+        cudaError_t e = cudaStreamIsCapturing(stream_, &st);
+        if (e != cudaSuccess || st != cudaStreamCaptureStatusNone) return e;
+        if ((e = cudaStreamWaitEvent(stream_, event_, 0)) == cudaSuccess) begun_ = true;
+        return e;
+    }
+    cudaError_t end()
+    {
+        if (!begun_) return cudaSuccess;
+        begun_ = false;
+        return cudaEventRecord(event_, stream_);
+    }
+    ~Turn() { end(); }
+
+private:
+    std::lock_guard<std::mutex> lock_;
+    cudaEvent_t event_;
+    cudaStream_t stream_;
+    bool begun_ = false;
+};
 
 // Number of reference-block positions along one axis: the clamped scan of
 // source/BM3D_Base.cpp:421-443 (0, step, 2*step, ..., then extent - B).
@@ -205,6 +239,8 @@ extern "C" BM3D_API int bm3d_basic_noalloc(const float *src, float *dst, int wid
     int *cnt = reinterpret_cast<int *>(base + o_cnt);
     int *sy = reinterpret_cast<int *>(base + o_sy), *sx = reinterpret_cast<int *>(base + o_sx);
 
+    Turn turn(dev, s);
+    if ((e = turn.begin()) != cudaSuccess) return set_error(BM3D_ERR_CUDA, cuda_text("wait for the call before", e));
     if ((e = cudaMemcpy2DAsync(S, (size_t)ld * 4, src, (size_t)stride, (size_t)width * 4, height, cudaMemcpyDeviceToDevice, s)) != cudaSuccess)
         return set_error(BM3D_ERR_CUDA, cuda_text("input copy", e));
     // the accumulators keep the previous call's sums: clear them
@@ -297,5 +333,6 @@ extern "C" BM3D_API int bm3d_basic_noalloc(const float *src, float *dst, int wid
     if ((e = launch_finalize(fa, 1, s)) != cudaSuccess) return set_error(BM3D_ERR_CUDA, cuda_text("normalisation", e));
     if ((e = cudaMemcpy2DAsync(dst, (size_t)stride, num, (size_t)ld * 4, (size_t)width * 4, height, cudaMemcpyDeviceToDevice, s)) != cudaSuccess)
         return set_error(BM3D_ERR_CUDA, cuda_text("output copy", e));
+    if ((e = turn.end()) != cudaSuccess) return set_error(BM3D_ERR_CUDA, cuda_text("end of the call", e));
     return BM3D_OK;
 }
