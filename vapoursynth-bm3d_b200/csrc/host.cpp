@@ -1163,7 +1163,10 @@ public:
                 at += 2 * fs * planes;
             }
     }
-    void clear_acc() { CU(cudaMemsetAsync(acc_buf.p, 0, acc_bytes, stream)); }
+    void clear_acc()
+    {
+        if (acc_bytes) CU(cudaMemsetAsync(acc_buf.p, 0, acc_bytes, stream));
+    }
 
     bool learned_matching() const { return learned && para.B == 8 && para.G >= 2 && para.G <= 32; }
 
@@ -1244,6 +1247,8 @@ public:
     void run_cf(long long ngroups, long long blocks_per_frame, const uint32_t *pos, const int *cnt,
                 bool v, const int *winb, const int *slot0, int slots, long long acc_stride)
     {
+        // V-BM3D with every sigma zero: no tables, nothing to add
+        if (!acc_bytes) return;
         CFArgs a{};
         const DeviceTables &dt = device_tables();
         DevBuf *refws = rdef ? ws_ref : ws_src;
