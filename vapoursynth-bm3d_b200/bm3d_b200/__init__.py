@@ -333,8 +333,8 @@ class FilterNode(VideoNode):
         return out[:3 * nb].reshape(3, nb)
 
     def bm_tc_counts(self):
-        """Precision-form block matching of the last call: (reference blocks that fell back to
-        exact distances for every candidate, CTAs whose tensor-core wait timed out)."""
+        """Full-search block matching of the last call: (reference blocks whose distance estimates did not settle
+        the list, so that every distance was computed exactly; always 0)."""
         fb, to = C.c_int64(0), C.c_int64(0)
         capi.lib().bm3d_debug_bm_tc_counts(self._h, C.byref(fb), C.byref(to))
         return int(fb.value), int(to.value)

@@ -109,8 +109,8 @@ struct BMArgs {
     uint32_t *out_pos;         // [frame][by][bx][G], packed (y << 16) | x
     int *out_n;                // [frame][by][bx]
     float *out_key;            // optional, [frame][by][bx][G]
-    unsigned long long *stats; // optional: [0] blocks that took the exact heap path, [1] precision
-                               // forms: blocks that needed an exact fallback, [2] tensor-core time-outs
+    unsigned long long *stats; // optional: [0] blocks that took the exact heap path, [1] blocks whose
+                               // estimates or proposals did not settle the list
     uint32_t *out_prop;        // optional (learned proposals): [frame][by][bx][nprop] candidate
                                // indices of each block's proposal set, unused slots 0xffffffff
     int warps;                 // warps per CTA

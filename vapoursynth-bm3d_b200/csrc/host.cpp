@@ -542,10 +542,10 @@ public:
     bool rdef = false;
     cudaStream_t stream = nullptr;
     cudaStream_t own = nullptr;
-    unsigned long long *stats = nullptr;      // [0] exact-heap selections, [1] precision-form matching
-                                              // fallbacks, [2] precision-form tensor-core time-outs
+    unsigned long long *stats = nullptr;      // [0] exact-heap selections, [1] blocks whose estimates or
+                                              // proposals did not settle the list
     unsigned long long last_slow = 0;
-    unsigned long long last_stats[3] = {0, 0, 0};
+    unsigned long long last_stats[2] = {0, 0};
     // stage timing (CUDA events on the filter's stream): 0 ingest, 1 block matching,
     // 2 predictive search, 3 collaborative filter + aggregation, 4 normalise / stack, 5 egress
     static constexpr int kStages = 6;
@@ -598,7 +598,7 @@ public:
     {
         CU(cudaStreamCreateWithFlags(&own, cudaStreamNonBlocking));
         stream = own;
-        CU(cudaMalloc(&stats, 3 * sizeof(unsigned long long)));
+        CU(cudaMalloc(&stats, 2 * sizeof(unsigned long long)));
     }
 
 protected:
@@ -1494,7 +1494,7 @@ public:
         }
         ensure_ws(count, count);
         ensure_acc(count);
-        CU(cudaMemsetAsync(stats, 0, 3 * sizeof(unsigned long long), stream));
+        CU(cudaMemsetAsync(stats, 0, 2 * sizeof(unsigned long long), stream));
         mark(0);
         std::vector<bool> full(count);
         for (int k = 0; k < count; ++k) full[k] = frame_full(*src[k]);
@@ -1666,7 +1666,7 @@ public:
         v_n.get(sizeof(int) * nb);
         v_key.get(sizeof(float) * nb * para.G);
         ensure_acc(acc_planes);
-        CU(cudaMemsetAsync(stats, 0, 3 * sizeof(unsigned long long), stream));
+        CU(cudaMemsetAsync(stats, 0, 2 * sizeof(unsigned long long), stream));
         // window frames into the workspace; properties of each output frame's own source frame
         std::vector<bool> full(nwin);
         for (int i = 0; i < nwin; ++i) full[i] = true;
@@ -2264,7 +2264,7 @@ BM3D_API int bm3d_debug_bm_tc_counts(bm3d_filter *h, int64_t *fallbacks, int64_t
 {
     if (!h) return -1;
     if (fallbacks) *fallbacks = (int64_t)h->f->last_stats[1];
-    if (timeouts) *timeouts = (int64_t)h->f->last_stats[2];
+    if (timeouts) *timeouts = 0;
     return 0;
 }
 

@@ -303,8 +303,9 @@ cudaError_t launch_cf_fast(const CFArgs &a, cudaStream_t s)
     const bool w = a.wiener != 0;
     switch (a.G) {
     case 8: return w ? launch_cf_fast_t<8, true>(a, s) : launch_cf_fast_t<8, false>(a, s);
-    case 16: return w ? launch_cf_fast_t<16, true>(a, s) : launch_cf_fast_t<16, false>(a, s);
-    case 32: return w ? launch_cf_fast_t<32, true>(a, s) : launch_cf_fast_t<32, false>(a, s);
+    // Wiener: only the short groups that the tensor-core kernel leaves, which takes all of these lengths
+    case 16: return w ? cudaErrorInvalidValue : launch_cf_fast_t<16, false>(a, s);
+    case 32: return w ? cudaErrorInvalidValue : launch_cf_fast_t<32, false>(a, s);
     default: return cudaErrorInvalidValue;
     }
 }
