@@ -573,7 +573,7 @@ __global__ void __launch_bounds__(NP * 64, 8 / NP) cf_box_kernel(CFArgs a, CFBox
 // the same place of slots A and B, through both directions of the transform.
 // Bound: the shared-memory pipe (random-row loads of the blocks, transposes, and four native atomics a
 // pixel pair: 6.7 k of a step's 25 k clocks are atomics).  1920x1080 RGB x 8, step 4, G = 16: 12.6 ms with
-// per-lane gathers and float atomics on the plane (cf_fast_kernel), 8.3 ms now.
+// per-lane gathers and float atomics on the plane (cf_fast_kernel), 8.6 ms now (8.3 ms on an absolute grid).
 
 // A term is a pixel over its group's kept count, so its size follows the clip's, and an absolute grid would keep
 // fewer bits of a clip of small values than fp32 sums do.  So
@@ -581,8 +581,9 @@ __global__ void __launch_bounds__(NP * 64, 8 / NP) cf_box_kernel(CFArgs a, CFBox
 //   of two: its terms are those of the clip, scaled;
 // - a group whose terms are still below kBoxMin (a dark part of a bright tile) goes to the plane directly, as
 //   blocks of large terms do.
-// The grid's rounding is then at most 2^-19 of the largest term of a group's first block, and usually far less: the
-// test takes one coefficient's share of it.  A pixel averages the roundings of dozens of terms.
+// The grid's rounding is then at most 2^-19 of the largest term of the group's first block (of its seventeenth for the
+// second warp of a group of 32), and usually far less: the test takes one coefficient's share of it.  A pixel
+// averages the roundings of dozens of terms.
 constexpr float kTileMin = 0.0625f;                                            // 2^-4
 constexpr float kBoxMin = 6.103515625e-5f;                                     // 2^-14
 
@@ -779,8 +780,7 @@ __global__ void __launch_bounds__(NP * 64, 8 / NP) cf_boxh_kernel(CFArgs a, CFBo
     int *acc = reinterpret_cast<int *>(tr + NP * kT);                  // high words, then low words
     float *box = reinterpret_cast<float *>(acc + 2 * cells);
     unsigned *tops = reinterpret_cast<unsigned *>(box + cells);        // [warp]
-    int *red = reinterpret_cast<int *>(tops + 2 * NP) + pair * 6 * GPW;  // [group of the slots][warp]: kept counts,
-    int *redA = red + 2 * GPW, *redB = redA + 2 * GPW;                 // magnitude bits of the first blocks of A and of B
+    int *red = reinterpret_cast<int *>(tops + 2 * NP) + pair * 2 * GPW;  // [group of the slots][warp]
     const float *src = a.src[p] + f * a.frame_stride;
     const int h = lane & 1;
     const int blk = 16 * role + (lane >> 1);        // the lane's block of a slot: group sub, place z
@@ -858,14 +858,7 @@ __global__ void __launch_bounds__(NP * 64, 8 / NP) cf_boxh_kernel(CFArgs a, CFBo
             const int ma = q < gA ? min(a.count[grpA + q], G) : 0, mb = q < gB ? min(a.count[grpB + q], G) : 0;
             const int at = pair * kT + q * G * kBT + col;
             const int kept = box_hard_pair<G>(at, a, p, fxy, ma, mb);
-            float ca, cb;
-            upk(reinterpret_cast<f2 *>(smem)[at], ca, cb);
-            const unsigned ta = __reduce_max_sync(0xffffffffu, abs_bits(ca)), tb0 = __reduce_max_sync(0xffffffffu, abs_bits(cb));
-            if (lane == 0) {
-                red[2 * q + role] = kept;
-                redA[2 * q + role] = (int)ta;
-                redB[2 * q + role] = (int)tb0;
-            }
+            if (lane == 0) red[2 * q + role] = kept;
         }
         pair_barrier(1 + pair);
         const int kept = red[2 * sub] + red[2 * sub + 1], kA = kept & 0xffff, kB = kept >> 16;
@@ -875,13 +868,33 @@ __global__ void __launch_bounds__(NP * 64, 8 / NP) cf_boxh_kernel(CFArgs a, CFBo
         }
         const float dA = kA < 1 ? 1.0f : __fdiv_rn(1.0f, (float)kA), dB = kB < 1 ? 1.0f : __fdiv_rn(1.0f, (float)kB);
         const float wA = actA ? __fdiv_rn(dA, a.amp[na - 1]) * up : 0.0f, wB = actB ? __fdiv_rn(dB, a.amp[nb - 1]) * up : 0.0f;
-        // a pixel is, on the mean square, at least as large as any one of the block's coefficients
-        const float tA = __int_as_float(max(redA[2 * sub], redA[2 * sub + 1])) * wA;
-        const float tB = __int_as_float(max(redB[2 * sub], redB[2 * sub + 1])) * wB;
-        const bool apartA = actA && tA > 0.0f && tA < kBoxMin, apartB = actB && tB > 0.0f && tB < kBoxMin;
-        const unsigned apart = __ballot_sync(0xffffffffu, apartA || apartB), places = __ballot_sync(0xffffffffu, actA || actB);
+        // largest coefficient of the first of the warp's blocks of the lane's group, by the lanes of that group
+        constexpr int kLanes = G < 16 ? 2 * G : 32;
+        unsigned ta = 0u, tb0 = 0u;
+#pragma unroll
+        for (int j = lane & (kLanes - 1); j < 64; j += kLanes) {
+            float u, w;
+            upk(tr[pair * kT + (16 * role + (lane & ~(kLanes - 1)) / 2) * kBT + j], u, w);
+            ta = max(ta, abs_bits(u));
+            tb0 = max(tb0, abs_bits(w));
+        }
+        __syncwarp();
         box_inverse2(tb, pk(wA, wB), actA, actB, h);
         __syncwarp();
+        if constexpr (kLanes == 32) {
+            ta = __reduce_max_sync(0xffffffffu, ta);
+            tb0 = __reduce_max_sync(0xffffffffu, tb0);
+        } else {
+#pragma unroll
+            for (int o = kLanes / 2; o > 0; o >>= 1) {
+                ta = max(ta, __shfl_xor_sync(0xffffffffu, ta, o));
+                tb0 = max(tb0, __shfl_xor_sync(0xffffffffu, tb0, o));
+            }
+        }
+        // a pixel is, on the mean square, at least as large as any one of its block's coefficients
+        const float tA = __uint_as_float(ta) * wA, tB = __uint_as_float(tb0) * wB;
+        const bool apartA = actA && tA > 0.0f && tA < kBoxMin, apartB = actB && tB > 0.0f && tB < kBoxMin;
+        const unsigned apart = __ballot_sync(0xffffffffu, apartA || apartB), places = __ballot_sync(0xffffffffu, actA || actB);
         // aggregation, four blocks (two places of both slots) per step
         const f2 *v = tr + pair * kT + 16 * role * kBT + lane;
         int *cell = acc + sy * P + sx, *cell0 = acc + sy * 8 + sx;

@@ -206,7 +206,7 @@ static bool cf_box_fit(const CFArgs &a, CFBox &g, int step, int G, size_t *smem)
             const int rows = std::min(a.H, 2 * g.range + 8 + (ny - 1) * step);
             const int pitch = w + ((12 - (w & 7)) & 7);      // 4 mod 8: a scatter step's eight rows in distinct banks
             const size_t bytes = (size_t)kBoxPairs * 32 * kBT * 8 + ((size_t)rows * pitch + 64) * cell +
-                                 (size_t)kBoxPairs * 2 * gpw * 4 * (a.wiener ? 1 : 3) + (a.wiener ? 0 : (size_t)kBoxPairs * 2 * 4);
+                                 (size_t)kBoxPairs * 2 * gpw * 4 + (a.wiener ? 0 : (size_t)kBoxPairs * 2 * 4);
             if (bytes > kBoxCap) break;
             const int slots = ny * (nx / gpw), steps = (slots + per_step - 1) / per_step;
             most = std::max(most, slots);
